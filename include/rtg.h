@@ -121,12 +121,13 @@ typedef struct rtg_launch_config {
   int32_t stack_depth;       /* traversal stack entries, 32, 64 or 256; 0 = the smallest that holds the
                                 tree (a smaller request than the tree needs is raised to that) */
   int32_t scheduling;        /* RTG_SCHED_* */
-  int32_t leaf_tests;        /* RTG_LEAF_*: when the primitives of a leaf the ray reaches are tested */
+  int32_t leaf_tests;        /* RTG_LEAF_*: accepted, no effect (see below) */
   int32_t stack_memory;      /* RTG_STACK_*: where the traversal stack of the path kernel lives */
 } rtg_launch_config;
-/* leaf_tests: on the spot, or postponed until every lane of the warp holds a
- * leaf (Aila and Laine's while-while traversal; megakernel and plain
- * schedules, forward traces) */
+/* leaf_tests: the primitives of a leaf are tested on the spot in either case.
+ * Postponing them until every lane of the warp holds a leaf (Aila and Laine's
+ * while-while traversal) was an option of the binary traversal; the four-box
+ * visits are faster than both, and waiting for the warp no longer pays. */
 #define RTG_LEAF_IMMEDIATE 0
 #define RTG_LEAF_POSTPONED 1
 /* stack_memory: per-thread local memory (cached in L1 beside the tree), or
@@ -204,22 +205,19 @@ RTG_API int rtg_set_tree_builder(rtg_context* ctx, int32_t builder);
 RTG_API int rtg_get_tree_builder(const rtg_context* ctx, int32_t* builder);
 /* Which tree the closest-hit queries traverse (no counterpart in rti; Embree
  * chooses its own):
- *   RTG_NODES_BINARY (2): the binary tree itself (64-byte nodes, both child
- *     boxes in float);
+ *   RTG_NODES_BINARY (2): the binary tree in float boxes, visited up to four
+ *     boxes at a time (128-byte nodes made by every build and refit);
  *   RTG_NODES_WIDE (8): a compressed 8-wide tree collapsed from it after every
  *     build and refit (96-byte nodes, child boxes as bytes on a per-node
  *     power-of-two grid, children ordered by direction).  Its boxes contain
  *     the binary boxes, so results are the same bit for bit;
- *   RTG_NODES_AUTO (0, the default): wide when the binary nodes and the
- *     primitive records outgrow the L2 cache, else binary.  Measured: the wide
- *     tree moves a third less DRAM traffic and traces a 4.19 M-disc surface
- *     13-16 % faster, but costs more instructions per query and traces
- *     L2-resident surfaces (200 k triangles, 98 k discs) 3-10 % slower.
+ *   RTG_NODES_AUTO (0, the default): as RTG_NODES_BINARY, the faster one on
+ *     every surface measured (4.19 M discs, beyond the L2 cache, 2e7 rays:
+ *     27 ms against 30.5 ms over the wide tree).
  * A scene with a node wider than 4080 units, or a wide tree whose traversal
  * stack would exceed 256 entries, is traced over the binary tree whatever this
- * says.  The postponed leaf tests (RTG_LEAF_POSTPONED) and the multi-hit
- * window's interval queries always use the binary tree.  rtg_autotune tries
- * both for its fastest candidates. */
+ * says.  The multi-hit window's interval queries always walk the binary tree.
+ * rtg_autotune sets RTG_NODES_BINARY. */
 #define RTG_NODES_AUTO 0
 #define RTG_NODES_BINARY 2
 #define RTG_NODES_WIDE 8
@@ -273,13 +271,12 @@ RTG_API int rtg_get_visit_limit(const rtg_context* ctx, uint64_t* visits);
  * context as it was. */
 RTG_API int rtg_inject_alloc_failure(rtg_context* ctx, int64_t after);
 /* Autotuner: for each tree builder (RTG_TREE_*), times each candidate launch
- * configuration (block size x packet x stack depth x leaf tests, megakernel
- * or plain; the wavefront schedule, slower on every workload measured, is
+ * configuration (block size x packet x stack depth, megakernel or plain; the wavefront schedule, slower on every workload measured, is
  * left to rtg_set_launch_config) on source
  * rays [0, sample_rays) with `seed` under the current surface and
- * configuration, over the node width RTG_NODES_AUTO picks; re-times the three
- * fastest of each tree with their stacks in the other memory and over the
- * other node width; keeps the fastest as the context's tree, node width and
+ * configuration, over RTG_NODES_BINARY; re-times the three fastest of each
+ * tree with their stacks in the other memory; keeps the fastest as the
+ * context's tree, node width and
  * launch configuration and returns the latter (best and best_rays_per_s may
  * be NULL; rtg_get_tree_builder and rtg_get_node_width tell the rest).  Leaves
  * no trace results behind (trace again afterwards). */

@@ -363,10 +363,9 @@ void drop_surface(rtg_context* ctx) {
   cudaStreamSynchronize(ctx->stream);
   Geometry& g = ctx->g;
   dfree(g.disc_cr_by_id); dfree(g.disc_n_by_id); dfree(g.tri_v); dfree(g.tri_idx);
-  dfree(g.disc); dfree(g.tri); dfree(g.nodes);
+  dfree(g.disc); dfree(g.tri); dfree(g.nodes); dfree(g.quads);
   dfree(g.leaf_ref); dfree(g.leaf_prim); dfree(g.parent); dfree(g.prim_lo); dfree(g.prim_hi);
   dfree(g.refit_flags); dfree(g.nb_ptr); dfree(g.nb_idx); dfree(g.nb_slot); dfree(g.disc_slot);
-  dfree(g.wnodes);
   dfree(g.wnodes);
   g.n_wnodes = 0;
   g.wide_stack = 0;
@@ -376,6 +375,7 @@ void drop_surface(rtg_context* ctx) {
   g.nb_nnz = 0;
   g.root = 0;
   g.depth = 0;
+  g.quad_stack = 0;
   ctx->traced = false;
   ctx->finalized = false;
   ++ctx->version;
@@ -529,11 +529,12 @@ int rtg_destroy(rtg_context* ctx) {
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   Geometry& g = ctx->g;
   dfree(g.disc_cr_by_id); dfree(g.disc_n_by_id); dfree(g.tri_v); dfree(g.tri_idx);
-  dfree(g.disc); dfree(g.tri); dfree(g.nodes);
+  dfree(g.disc); dfree(g.tri); dfree(g.nodes); dfree(g.quads);
   dfree(g.leaf_ref); dfree(g.leaf_prim); dfree(g.parent); dfree(g.prim_lo); dfree(g.prim_hi);
   dfree(g.refit_flags); dfree(g.nb_ptr); dfree(g.nb_idx); dfree(g.nb_slot); dfree(g.disc_slot);
   dfree(ctx->sticking_field); dfree(ctx->acc); dfree(ctx->cnt); dfree(ctx->areas); dfree(ctx->est);
   dfree(ctx->stat_tmp);
+  dfree(g.wnodes);
   dfree(ctx->seglog);
   dfree(ctx->seglog_count);
   free_wavefront(ctx->wf);
@@ -904,19 +905,18 @@ static int rtg_autotune_body(rtg_context* ctx, uint64_t sample_rays, uint64_t se
     if (rc == RTG_OK) rc = prepare_trace(ctx, 0, sample_rays, seed, p);  // the tree changed
     if (rc != RTG_OK) break;
     const size_t first = cand.size();
-    const int32_t width = outgrows_l2(ctx) ? RTG_NODES_WIDE : RTG_NODES_BINARY;  // the automatic choice
+    const int32_t width = RTG_NODES_BINARY;  // the automatic choice
     // the wavefront schedule is not a candidate: its queue traffic lost to the
     // megakernel on every workload measured (it stays selectable by hand)
     for (int sched : {RTG_SCHED_MEGAKERNEL, RTG_SCHED_PLAIN})
       for (int tpb : {64, 128, 256})
         for (int packet : {1, 8, 32})
-          for (int stack : {0, 256})
-            for (int leaf : {RTG_LEAF_IMMEDIATE, RTG_LEAF_POSTPONED}) {
-              if (sched == RTG_SCHED_PLAIN && (packet != 1 || tpb == 64 || stack != 0)) continue;
-              if (stack == 256 && stack_for(0, traversal_depth(ctx)) == 256) continue;
-              if (leaf == RTG_LEAF_POSTPONED && packet == 32) continue;
-              cand.push_back(Cand{builder, width, rtg_launch_config{tpb, packet, stack, sched, leaf, RTG_STACK_AUTO}, 0.0f});
-            }
+          for (int stack : {0, 256}) {
+            if (sched == RTG_SCHED_PLAIN && (packet != 1 || tpb == 64 || stack != 0)) continue;
+            if (stack == 256 && stack_for(0, traversal_depth(ctx)) == 256) continue;
+            cand.push_back(Cand{builder, width,
+                                rtg_launch_config{tpb, packet, stack, sched, RTG_LEAF_IMMEDIATE, RTG_STACK_AUTO}, 0.0f});
+          }
     float ms = 0.0f;
     for (size_t i = first; i < cand.size() && rc == RTG_OK; ++i) {
       rc = run(cand[i], ms);  // warm-up
@@ -944,19 +944,6 @@ static int rtg_autotune_body(rtg_context* ctx, uint64_t sample_rays, uint64_t se
         cand.push_back(alt);
       }
     }
-    // the three fastest over the other tree layout (binary / wide), best of two
-    if (ctx->g.n_wnodes > 0)
-      for (size_t q = 0; q < order.size() && q < 3 && rc == RTG_OK; ++q) {
-        Cand alt = cand[order[q]];
-        alt.width = alt.width == RTG_NODES_WIDE ? RTG_NODES_BINARY : RTG_NODES_WIDE;
-        float m2 = 0.0f;
-        rc = run(alt, alt.ms);
-        if (rc == RTG_OK) rc = run(alt, m2);
-        if (rc == RTG_OK) {
-          alt.ms = std::min(alt.ms, m2);
-          cand.push_back(alt);
-        }
-      }
   }
   ctx->traced = false;
   ctx->finalized = false;

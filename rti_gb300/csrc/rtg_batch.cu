@@ -439,13 +439,11 @@ static int rtg_batch_autotune_body(rtg_batch* b, double fraction, rtg_launch_con
   for (int sched : {RTG_SCHED_MEGAKERNEL, RTG_SCHED_PLAIN})
     for (int tpb : {64, 128, 256})
       for (int packet : {1, 8, 32})
-        for (int stack : {0, 256})
-          for (int leaf : {RTG_LEAF_IMMEDIATE, RTG_LEAF_POSTPONED}) {
-            if (sched == RTG_SCHED_PLAIN && (packet != 1 || tpb == 64 || stack != 0)) continue;
-            if (stack == 256 && stack_for(0, b->depth) == 256) continue;
-            if (leaf == RTG_LEAF_POSTPONED && packet == 32) continue;
-            cand.push_back(rtg_launch_config{tpb, packet, stack, sched, leaf, RTG_STACK_AUTO});
-          }
+        for (int stack : {0, 256}) {
+          if (sched == RTG_SCHED_PLAIN && (packet != 1 || tpb == 64 || stack != 0)) continue;
+          if (stack == 256 && stack_for(0, b->depth) == 256) continue;
+          cand.push_back(rtg_launch_config{tpb, packet, stack, sched, RTG_LEAF_IMMEDIATE, RTG_STACK_AUTO});
+        }
   std::vector<float> tms(cand.size(), 0.0f);
   float ms = 0.0f;
   for (size_t i = 0; i < cand.size() && rc == RTG_OK; ++i) {

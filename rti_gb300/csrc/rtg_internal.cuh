@@ -17,7 +17,10 @@ namespace rtg {
 constexpr uint32_t kLeafBit = 0x80000000u;
 constexpr uint32_t kTriBit = 0x40000000u;
 constexpr uint32_t kSlotMask = 0x3FFFFFFFu;
-constexpr int kStackSize = 64;
+// deepest binary tree kept (the radix tree's depth is bounded by its 62 key
+// bits; a clustering deeper than this falls back to it): the largest traversal
+// stack holds 256 entries, and a quad's can exceed the binary one by 64
+constexpr int kMaxDepth = 192;
 
 // One internal node: the boxes of both children and their references (64 B).
 //   a = (c0.lo.x, c0.hi.x, c1.lo.x, c1.hi.x)
@@ -29,8 +32,27 @@ struct __align__(16) Node {
   uint4 d;
 };
 
-// One node of the compressed 8-wide tree the closest-hit query traverses
-// (collapsed from the binary LBVH after every build and refit; rtg_wide.cu).
+// One node as the closest-hit query visits it: up to four boxes below a binary
+// node (its children, the larger ones opened; rtg_lbvh.cu) as centre and half
+// extent, 128 B, at the binary node's index.  The pairs are operands of
+// two-wide float instructions: x and y of one child, or z of two.
+//   xy[k] = (centre.x, centre.y, half.x, half.y) of child k
+//   z[j]  = (centre.z of 2j, of 2j + 1, half.z of 2j, of 2j + 1)
+//   ref   = the children's references; a missing child has half extents -1e30
+//           (a box that no ray meets)
+// The half extents are rounded up and widened by 2^-20 of themselves and 2^-21
+// of the centre, which covers the rounding of the slab test (quad_test in
+// rtg_path.cuh) for rays that start near the box; the test's relative slack
+// covers it far away.
+struct __align__(128) QuadNode {
+  float4 xy[4];
+  float4 z[2];
+  uint4 ref;
+  uint4 unused;
+};
+
+// One node of the compressed 8-wide tree the closest-hit query may traverse
+// instead (RTG_NODES_WIDE; collapsed from the binary LBVH after every build and refit; rtg_wide.cu).
 // 96 bytes, read by three 256-bit loads:
 //   w[0..2]  node origin p (float bits), an exact multiple of the axis quantum
 //   w[3]     biased exponents e_x, e_y, e_z of the quanta 2^e (bytes 0..2) and
@@ -69,10 +91,11 @@ struct SceneView {
   // triangles in slot order, 64 B each: (v0, original id bits), e1, e2, unit normal
   const float4* tri;
   int32_t nt;
-  const Node* nodes;
+  const Node* nodes;       // the binary tree (the window deposit's interval queries)
+  const QuadNode* quads;   // the same tree as closest hits visit it, up to four boxes a node
   uint32_t root;        // child reference of the root (internal node 0 or a leaf)
   // the 8-wide compressed tree of the closest-hit query (root = wide node 0),
-  // or nullptr: closest hits traverse the binary nodes
+  // or nullptr: closest hits visit the quads
   const WideNode* wnodes;
   uint32_t n_wnodes;
   // neighbour CSR: rows by original disc id, columns as disc slots (the
@@ -156,6 +179,7 @@ struct Geometry {
   DBuf<float4> disc;       // 2 per slot: (centre, radius), (normal, id bits)
   DBuf<float4> tri;        // 4 per slot: (v0, id bits), e1, e2, unit normal
   DBuf<Node> nodes;
+  DBuf<QuadNode> quads;
   DBuf<uint32_t> leaf_ref;    // per sorted leaf i: child reference
   DBuf<int32_t> leaf_prim;    // per sorted leaf i: original primitive id
   DBuf<uint32_t> parent;      // parent of internal nodes [0,n-1) and leaves [n-1, 2n-1)
@@ -173,6 +197,7 @@ struct Geometry {
   float rmax = 0.0f;
   float tri_min[3] = {0, 0, 0}, tri_max[3] = {0, 0, 0};
   int32_t depth = 0;  // internal nodes on the longest root-to-leaf path
+  int32_t quad_stack = 0;  // traversal stack entries the quads can need
   int32_t builder = 0;  // kBuilderKarras or kBuilderPloc
   // 8-wide compressed tree (rtg_wide.cu)
   DBuf<WideNode> wnodes;

@@ -13,7 +13,8 @@
 // leaves (build_ploc), whose trees need fewer node visits per query.
 //
 // Leaves hold one primitive; each internal node stores the boxes of both
-// children (64 bytes), so one node fetch decides both children.
+// children (64 bytes).  Closest hits visit QuadNodes instead, which the refit
+// makes on its way up: up to four boxes below the node in one fetch.
 #include <cfloat>
 #include <cstdint>
 #include <vector>
@@ -504,11 +505,113 @@ __device__ __forceinline__ void child_box(uint32_t ref, const float4* __restrict
   }
 }
 
-// Bottom-up refit: the second thread to reach a node writes both child boxes.
+// A box as a QuadNode stores it.
+struct QuadBox {
+  float c[3], h[3];
+};
+__device__ __forceinline__ QuadBox quad_box(const float* lo, const float* hi) {
+  QuadBox q;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    q.c[a] = 0.5f * lo[a] + 0.5f * hi[a];
+    const float e = fmaxf(__fsub_ru(hi[a], q.c[a]), __fsub_ru(q.c[a], lo[a]));
+    q.h[a] = __fadd_ru(__fmul_ru(e, 1.00000096f), __fmul_ru(fabsf(q.c[a]), 0x1p-21f));
+  }
+  return q;
+}
+
+// What a traversal from a node can need: the low half is the stack entries
+// (inner children but one wait while one is descended into), the high half the
+// node's height in binary levels.
+constexpr int kNeedShift = 16;
+
+// The QuadNode of a binary node from its two children, whose own nodes are
+// complete: as long as there is room, the child of largest surface area is
+// opened, which saves the query a visit.  Opening stops where the stack could
+// outgrow the binary tree's by more than 64 entries (kMaxDepth leaves room for
+// them).  Returns the node's need.
+__device__ int32_t make_quad(QuadNode* out, const Node* nodes, const int32_t* need, uint4 d, const float* l0,
+                             const float* h0, const float* l1, const float* h1) {
+  int32_t height = 0;
+  if (!(d.x & kLeafBit)) height = __ldcg(&need[d.x]) >> kNeedShift;
+  if (!(d.y & kLeafBit)) height = max(height, __ldcg(&need[d.y]) >> kNeedShift);
+  height += 1;
+  float lo[4][3], hi[4][3];
+  uint32_t ref[4];
+  int n = 0;
+  int32_t stack = 0;
+  for (int most = 4; most >= 2; most -= 2) {
+    for (int a = 0; a < 3; ++a) {
+      lo[0][a] = l0[a];
+      hi[0][a] = h0[a];
+      lo[1][a] = l1[a];
+      hi[1][a] = h1[a];
+    }
+    ref[0] = d.x;
+    ref[1] = d.y;
+    n = d.x == d.y ? 1 : 2;  // a one-primitive tree holds its leaf in both children of the root
+    while (n > 1 && n < most) {
+      int best = -1;
+      float ba = -1.0f;
+      for (int k = 0; k < n; ++k) {
+        if (ref[k] & kLeafBit) continue;
+        const float x = hi[k][0] - lo[k][0], y = hi[k][1] - lo[k][1], z = hi[k][2] - lo[k][2];
+        const float area = x * y + y * z + z * x;
+        if (area > ba) {
+          ba = area;
+          best = k;
+        }
+      }
+      if (best < 0) break;
+      const Node* o = nodes + ref[best];
+      const float4 a = __ldcg(&o->a), b = __ldcg(&o->b), c = __ldcg(&o->c);
+      const uint4 r = __ldcg(&o->d);
+      const float box0[6] = {a.x, b.x, c.x, a.y, b.y, c.y}, box1[6] = {a.z, b.z, c.z, a.w, b.w, c.w};
+      for (int k = 0; k < 3; ++k) {
+        lo[best][k] = box0[k];
+        hi[best][k] = box0[3 + k];
+        lo[n][k] = box1[k];
+        hi[n][k] = box1[3 + k];
+      }
+      ref[best] = r.x;
+      ref[n] = r.y;
+      ++n;
+    }
+    int inner = 0, deepest = 0;
+    for (int k = 0; k < n; ++k)
+      if (!(ref[k] & kLeafBit)) {
+        inner += 1;
+        deepest = max(deepest, __ldcg(&need[ref[k]]) & ((1 << kNeedShift) - 1));
+      }
+    stack = inner > 0 ? deepest + inner - 1 : 0;
+    if (stack <= height + 64) break;
+  }
+  QuadBox q[4];
+  for (int k = 0; k < 4; ++k) {
+    if (k < n) {
+      q[k] = quad_box(lo[k], hi[k]);
+    } else {
+      ref[k] = d.x;
+      for (int a = 0; a < 3; ++a) {
+        q[k].c[a] = 0.0f;
+        q[k].h[a] = -1e30f;
+      }
+    }
+    out->xy[k] = make_float4(q[k].c[0], q[k].c[1], q[k].h[0], q[k].h[1]);
+  }
+  out->z[0] = make_float4(q[0].c[2], q[1].c[2], q[0].h[2], q[1].h[2]);
+  out->z[1] = make_float4(q[2].c[2], q[3].c[2], q[2].h[2], q[3].h[2]);
+  out->ref = make_uint4(ref[0], ref[1], ref[2], ref[3]);
+  return stack | (height << kNeedShift);
+}
+
+// Bottom-up refit: the second thread to reach a node writes both child boxes
+// and the node's QuadNode.
 __global__ void refit_kernel(int64_t n, const uint32_t* __restrict__ leaf_ref, const uint32_t* __restrict__ parent,
                              const float4* __restrict__ dn, const float4* __restrict__ tri,
                              const float* __restrict__ plo, const float* __restrict__ phi, Node* nodes,
-                             float* node_box, unsigned int* flags, unsigned long long* errors) {
+                             QuadNode* quads, float* node_box, int32_t* need, unsigned int* flags,
+                             unsigned long long* status) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   uint32_t node = parent[(n - 1) + i];
@@ -529,11 +632,15 @@ __global__ void refit_kernel(int64_t n, const uint32_t* __restrict__ leaf_ref, c
       node_box[6 * (int64_t)node + a] = fminf(l0[a], l1[a]);
       node_box[6 * (int64_t)node + 3 + a] = fmaxf(h0[a], h1[a]);
     }
+    need[node] = make_quad(quads + node, nodes, need, r, l0, h0, l1, h1);
     __threadfence();
-    if (node == 0) return;
+    if (node == 0) {
+      status[1] = (unsigned long long)(need[0] & ((1 << kNeedShift) - 1));
+      return;
+    }
     node = parent[node];
   }
-  atomicAdd(errors, 1ull);
+  atomicAdd(&status[0], 1ull);
 }
 
 // Structural check of the tree before any traversal: every child reference is
@@ -577,10 +684,11 @@ __global__ void count_check_kernel(const unsigned int* __restrict__ c, int64_t n
 
 __global__ void single_leaf_kernel(const uint32_t* __restrict__ leaf_ref, const float4* __restrict__ dn,
                                    const float4* __restrict__ tri, const float* __restrict__ plo,
-                                   const float* __restrict__ phi, Node* nodes) {
+                                   const float* __restrict__ phi, Node* nodes, QuadNode* quads) {
   uint32_t r = leaf_ref[0];
   float l[3], h[3];
   child_box(r, dn, tri, plo, phi, nullptr, l, h);
+  make_quad(quads, nodes, nullptr, make_uint4(r, r, 0u, 0u), l, h, l, h);
   nodes[0].a = make_float4(l[0], h[0], l[0], h[0]);
   nodes[0].b = make_float4(l[1], h[1], l[1], h[1]);
   nodes[0].c = make_float4(l[2], h[2], l[2], h[2]);
@@ -625,7 +733,7 @@ int tree_depth(rtg_context* ctx, cudaStream_t st) {
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   tfree(dd, st);
   if (e != cudaSuccess) return check_cuda(ctx, e, "tree depth");
-  if (h > 256) return set_error(ctx, RTG_ERR_INTERNAL, "LBVH deeper than 256 levels");
+  if (h > (unsigned)kMaxDepth) return set_error(ctx, RTG_ERR_INTERNAL, "LBVH deeper than 192 levels");
   g.depth = (int32_t)h;
   return RTG_OK;
 }
@@ -772,34 +880,40 @@ int run_slots_and_refit(rtg_context* ctx, const uint32_t* d_sorted_prim, const u
     RTG_CUDA(ctx, cudaGetLastError());
   }
   if (np == 1) {
-    single_leaf_kernel<<<1, 1, 0, st>>>(g.leaf_ref.p, g.disc.p, g.tri.p, g.prim_lo.p, g.prim_hi.p, g.nodes.p);
+    RTG_TRY(dalloc(ctx, g.quads, 1, "quad nodes"));
+    single_leaf_kernel<<<1, 1, 0, st>>>(g.leaf_ref.p, g.disc.p, g.tri.p, g.prim_lo.p, g.prim_hi.p, g.nodes.p,
+                                        g.quads.p);
     RTG_CUDA(ctx, cudaGetLastError());
+    g.quad_stack = 0;
     g.wide_current = false;
     return wants_wide(ctx) ? build_wide(ctx, st) : RTG_OK;
   }
   DBuf<float> node_box;
-  DBuf<unsigned long long> err;
+  DBuf<int32_t> need;
+  DBuf<unsigned long long> status;  // [0] errors, [1] stack entries the root's quad can need
   int rc = talloc(ctx, node_box, (size_t)(6 * (np - 1)), st, "node boxes");
-  if (rc == RTG_OK) rc = talloc(ctx, err, 1, st, "refit status");
+  if (rc == RTG_OK) rc = talloc(ctx, need, (size_t)(np - 1), st, "stack needs");
+  if (rc == RTG_OK) rc = talloc(ctx, status, 2, st, "refit status");
   if (rc == RTG_OK) rc = dalloc(ctx, g.refit_flags, (size_t)(np - 1), "refit flags");
+  if (rc == RTG_OK) rc = dalloc(ctx, g.quads, (size_t)(np - 1), "quad nodes");
+  auto cleanup = [&]() { tfree(node_box, st); tfree(need, st); tfree(status, st); };
   if (rc != RTG_OK) {
-    tfree(node_box, st);
-    tfree(err, st);
+    cleanup();
     return rc;
   }
   cudaMemsetAsync(g.refit_flags.p, 0, sizeof(unsigned int) * (np - 1), st);
-  cudaMemsetAsync(err.p, 0, sizeof(unsigned long long), st);
+  cudaMemsetAsync(status.p, 0, 2 * sizeof(unsigned long long), st);
   refit_kernel<<<blocks_for(np, 256), 256, 0, st>>>(np, g.leaf_ref.p, g.parent.p, g.disc.p, g.tri.p,
-                                                    g.prim_lo.p, g.prim_hi.p, g.nodes.p, node_box.p,
-                                                    g.refit_flags.p, err.p);
+                                                    g.prim_lo.p, g.prim_hi.p, g.nodes.p, g.quads.p, node_box.p,
+                                                    need.p, g.refit_flags.p, status.p);
   cudaError_t e = cudaGetLastError();
-  unsigned long long herr = 0;
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&herr, err.p, sizeof herr, cudaMemcpyDeviceToHost, st);
+  unsigned long long h[2] = {0, 0};
+  if (e == cudaSuccess) e = cudaMemcpyAsync(h, status.p, sizeof h, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  tfree(node_box, st);
-  tfree(err, st);
+  cleanup();
   if (e != cudaSuccess) return check_cuda(ctx, e, "LBVH refit");
-  if (herr) return set_error(ctx, RTG_ERR_INTERNAL, "LBVH refit exceeded its depth limit");
+  if (h[0]) return set_error(ctx, RTG_ERR_INTERNAL, "LBVH refit exceeded its depth limit");
+  g.quad_stack = (int32_t)h[1];
   g.wide_current = false;  // the wide tree's boxes follow the binary ones: now, or before a trace that wants it
   return wants_wide(ctx) ? build_wide(ctx, st) : RTG_OK;
 }

@@ -11,12 +11,12 @@
 // source-ray ids from a global counter (one atomic per warp), so long and
 // short paths share the SIMD lanes.
 //
-// Closest hit = stack traversal of the two-box LBVH nodes; ties in t go to the
-// lower primitive id, and the node boxes are conservative, so the chosen hit
-// does not depend on the traversal order.  The stack holds STACK entries (in
-// local memory, or in shared memory with one column per thread); a tree
-// deeper than that would overflow it (counted as an error), so the host picks
-// STACK from the tree depth.
+// Closest hit = stack traversal of the tree's four-box nodes; ties in t go to
+// the lower primitive id, and the node boxes are conservative, so the chosen
+// hit does not depend on the traversal order.  The stack holds STACK entries
+// (in local memory, or in shared memory with one column per thread); a tree
+// that needs more would overflow it (counted as an error), so the host picks
+// STACK from the tree's need.
 #pragma once
 #include <cfloat>
 #include <climits>
@@ -70,15 +70,82 @@ struct Ray {
   f3 o, d, idr;
 };
 
-// Slab test of one child box; returns the entry distance in tn.
-__device__ __forceinline__ bool slab(float lx, float hx, float ly, float hy, float lz, float hz, const Ray& r,
-                                     float tmax, float& tn) {
-  float t0x = (lx - r.o.x) * r.idr.x, t1x = (hx - r.o.x) * r.idr.x;
-  float t0y = (ly - r.o.y) * r.idr.y, t1y = (hy - r.o.y) * r.idr.y;
-  float t0z = (lz - r.o.z) * r.idr.z, t1z = (hz - r.o.z) * r.idr.z;
-  tn = max3f(fminf(t0x, t1x), fminf(t0y, t1y), fmaxf(fminf(t0z, t1z), 0.0f));
-  float tf = min3f(fmaxf(t0x, t1x), fmaxf(t0y, t1y), fmaxf(t0z, t1z));
-  return tn <= tf * 1.0000005f && tn <= tmax * 1.0000005f + 1e-30f;
+// Two-wide float arithmetic (sm_100+): each half is one IEEE operation, and a
+// pair takes one issue slot.
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 pack2(float x, float y) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f2 v, float& x, float& y) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v));
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ void load_pairs(const void* p, f2& a, f2& b, f2& c, f2& d) {  // 256 bits
+  asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(d) : "l"(p));
+}
+
+// A ray against boxes given as centre and half extent: per axis t of the
+// centre is c / d - o / d, and the slab reaches half / |d| to either side of it.
+struct QuadRay {
+  f2 ixy, izz;  // 1 / d (z twice)
+  f2 axy, azz;  // |1 / d|
+  f2 mxy, mzz;  // -|1 / d|
+  f2 nxy, nzz;  // -o / d
+};
+__device__ __forceinline__ QuadRay quad_ray(const Ray& r) {
+  QuadRay q;
+  q.ixy = pack2(r.idr.x, r.idr.y);
+  q.izz = pack2(r.idr.z, r.idr.z);
+  q.axy = pack2(fabsf(r.idr.x), fabsf(r.idr.y));
+  q.azz = pack2(fabsf(r.idr.z), fabsf(r.idr.z));
+  q.mxy = pack2(-fabsf(r.idr.x), -fabsf(r.idr.y));
+  q.mzz = pack2(-fabsf(r.idr.z), -fabsf(r.idr.z));
+  q.nxy = pack2(-r.o.x * r.idr.x, -r.o.y * r.idr.y);
+  q.nzz = pack2(-r.o.z * r.idr.z, -r.o.z * r.idr.z);
+  return q;
+}
+
+// The four boxes of a node: hit[k] where the ray meets box k within
+// [tmin, tmax], tn[k] where it enters.  18 two-wide FMAs and no minimum or
+// maximum per slab (lo/hi planes take 24 subtractions, 24 multiplications and
+// 24 minima for as many boxes).  The boxes' margins cover the rounding for a
+// ray that starts near them, the factor 1 + 2^-20 (over eight roundings of
+// 2^-24) for one far away, so a box that holds an accepted hit in
+// [tmin, tmax] is never missed.
+__device__ __forceinline__ void quad_test(const QuadNode* nd, const QuadRay& q, float tmin, float tmax, bool* hit,
+                                          float* tn, uint32_t* ref) {
+  const char* p = reinterpret_cast<const char*>(nd);
+  f2 c[4], e[4], cz[2], ez[2];
+  load_pairs(p, c[0], e[0], c[1], e[1]);
+  load_pairs(p + 32, c[2], e[2], c[3], e[3]);
+  load_pairs(p + 64, cz[0], ez[0], cz[1], ez[1]);
+  const uint4 r = __ldg(&nd->ref);
+  ref[0] = r.x;
+  ref[1] = r.y;
+  ref[2] = r.z;
+  ref[3] = r.w;
+  float nz[4], fz[4];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const f2 t = fma2(cz[k], q.izz, q.nzz);
+    unpack2(fma2(ez[k], q.mzz, t), nz[2 * k], nz[2 * k + 1]);
+    unpack2(fma2(ez[k], q.azz, t), fz[2 * k], fz[2 * k + 1]);
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const f2 t = fma2(c[k], q.ixy, q.nxy);
+    float nx, ny, fx, fy;
+    unpack2(fma2(e[k], q.mxy, t), nx, ny);
+    unpack2(fma2(e[k], q.axy, t), fx, fy);
+    tn[k] = max3f(nx, ny, fmaxf(nz[k], tmin));
+    hit[k] = tn[k] <= min3f(fx, fy, fz[k]) * 1.000001f && tn[k] <= tmax;
+  }
 }
 
 // One 64-B node as two 256-bit read-only loads (sm_100+ vector width; the
@@ -239,20 +306,27 @@ __device__ __forceinline__ bool closest_hit_wide(const SceneView& s, const Ray& 
 }
 
 // Closest primitive hit; returns false when nothing is hit.  errs counts
-// stack overflows and iteration-limit trips (both end the query).
-// POSTPONE = false: a leaf child whose box the ray enters is tested on the
-// spot.  POSTPONE = true (Aila and Laine, HPG 2009, "while-while"): a lane
-// keeps one such leaf pending and walks on through inner nodes until every
-// lane of the warp holds a pending leaf (or has no inner node left), then the
-// warp tests the pending leaves together; the closest hit is the same, only
-// the lanes that run the primitive tests together change.
+// stack overflows and visit-limit trips (both end the query).
+// Bound by instructions at low SIMD efficiency (6 of 32 lanes on the hole: the
+// lanes wait for the longest query of their warp, leaf tests run for two lanes
+// at a time) and by the chain of dependent loads and instructions in the tail.
+// Up to four boxes a visit (QuadNode): half the dependent loads of a visit per
+// binary node, and about the same instructions.  One launch, before (binary
+// nodes, lo/hi planes) and now: trench 1e6 rays 3.13 -> 2.23 ms, hole (200 k
+// triangles) 1e6 rays 17.7 -> 13.8 and 1e7 rays 52.2 -> 47.2, 2e7 rays onto
+// 4.19 M discs 30.5 (8-wide tree) -> 27.6.
+// Boxes that the ray leaves before tnear are skipped, since a hit
+// needs t > tnear: a ray that starts on a flat face passes over the whole face.
+// Leaf children hit are tested on the spot; of the inner ones the nearest is
+// visited next and the others wait on the stack, nearly sorted (near child of
+// each pair, then the near pair).
 // SST = 0: the stack is a per-thread local array; SST > 0: it is a column of
 // shared memory, entry i at sstk[i * SST] (SST = the block size, so the lanes
 // of a warp always hit distinct banks).
-// WIDE = false: the binary tree only (the wide traversal is not compiled in,
-// which keeps the binary kernels' registers); WIDE = true: the wide tree
-// whenever the scene view carries one.
-template <int STACK, bool POSTPONE, int SST = 0, bool WIDE = true, typename Count = unsigned long long>
+// WIDE = false: the quads only (the wide traversal is not compiled in, which
+// saves registers); WIDE = true: the wide tree whenever the scene view
+// carries one.
+template <int STACK, int SST = 0, bool WIDE = true, typename Count = unsigned long long>
 __device__ bool closest_hit(const SceneView& s, f3 o, f3 d, float tnear, float& bt, int& bid, uint32_t& bref,
                             Count& errs, uint32_t* sstk = nullptr) {
   Ray r;
@@ -263,119 +337,56 @@ __device__ bool closest_hit(const SceneView& s, f3 o, f3 d, float tnear, float& 
   bid = INT_MAX;
   bref = 0xFFFFFFFFu;
   uint32_t lstack[SST ? 1 : STACK];
-  if constexpr (WIDE && !POSTPONE) {
+  if constexpr (WIDE) {
     if (s.wnodes) return closest_hit_wide<STACK, SST>(s, r, tnear, bt, bid, bref, errs, lstack, sstk);
   }
   auto stack = [&](int i) -> uint32_t& { return SST ? sstk[i * SST] : lstack[i]; };
   int sp = 0;
   uint32_t cur = s.root;
   const uint32_t max_iter = s.max_visits;
-  if (!POSTPONE) {
-    for (uint32_t it = 0;; ++it) {
-      if (it >= max_iter) {
-        errs += 1;
-        break;
-      }
-      if (kChecked && !node_in_range(s, cur)) {
-        errs += 1;
-        break;
-      }
-      float4 a, b, c;
-      uint4 ch;
-      load_node(s.nodes + cur, a, b, c, ch);
-      float tn0, tn1;
-      bool h0 = slab(a.x, a.y, b.x, b.y, c.x, c.y, r, bt, tn0);
-      bool h1 = slab(a.z, a.w, b.z, b.w, c.z, c.w, r, bt, tn1);
-      // The leaf children go through one code path, so the lanes with a leaf
-      // at child 0 and those with one at child 1 test together (a warp runs
-      // the test once per node step, twice only where a lane has two leaves).
-      const bool l0 = h0 && (ch.x & kLeafBit), l1 = h1 && (ch.y & kLeafBit);
-      uint32_t lf = l0 ? ch.x : (l1 ? ch.y : kNoLeaf);
-      uint32_t lf2 = l0 && l1 ? ch.y : kNoLeaf;
-      while (lf != kNoLeaf) {
-        if (!kChecked || leaf_in_range(s, lf)) test_leaf(s, lf, r, tnear, bt, bid, bref);
-        else errs += 1;
-        lf = lf2;
-        lf2 = kNoLeaf;
-      }
-      h0 = h0 && !l0;
-      h1 = h1 && !l1;
-      if (h0 && h1) {
-        uint32_t nearc = tn0 <= tn1 ? ch.x : ch.y;
-        uint32_t farc = tn0 <= tn1 ? ch.y : ch.x;
-        if (sp < STACK) {
-          stack(sp++) = farc;
-        } else {
-          errs += 1;
-        }
-        cur = nearc;
-      } else if (h0) {
-        cur = ch.x;
-      } else if (h1) {
-        cur = ch.y;
-      } else {
-        if (sp == 0) break;
-        cur = stack(--sp);
-      }
+  const QuadRay qr = quad_ray(r);
+  const float tmin = tnear * 0.999999f;
+  for (uint32_t it = 0;; ++it) {
+    if (it >= max_iter || (kChecked && !node_in_range(s, cur))) {
+      errs += 1;
+      break;
     }
-    return bid != INT_MAX;
-  }
-  // while-while: leaves travel through `cur` and the stack like inner nodes
-  constexpr uint32_t kNone = 0xFFFFFFFFu;
-  uint32_t leaf = kNone;
-  uint32_t it = 0;
-  auto pop = [&]() -> uint32_t { return sp > 0 ? stack(--sp) : kNone; };
-  while (cur != kNone) {
-    // inner nodes until every lane of the warp holds a pending leaf
-    while (cur != kNone && !(cur & kLeafBit)) {
-      if (it++ >= max_iter) {
-        errs += 1;
-        cur = kNone;
-        break;
-      }
-      if (kChecked && !node_in_range(s, cur)) {
-        errs += 1;
-        cur = kNone;
-        break;
-      }
-      float4 a, b, c;
-      uint4 ch;
-      load_node(s.nodes + cur, a, b, c, ch);
-      float tn0, tn1;
-      const bool h0 = slab(a.x, a.y, b.x, b.y, c.x, c.y, r, bt, tn0);
-      const bool h1 = slab(a.z, a.w, b.z, b.w, c.z, c.w, r, bt, tn1);
-      if (h0 && h1) {
-        const bool first = tn0 <= tn1;
-        if (sp < STACK) stack(sp++) = first ? ch.y : ch.x;
-        else errs += 1;
-        cur = first ? ch.x : ch.y;
-      } else if (h0) {
-        cur = ch.x;
-      } else if (h1) {
-        cur = ch.y;
-      } else {
-        cur = pop();
-      }
-      if (cur != kNone && (cur & kLeafBit) && leaf == kNone) {
-        leaf = cur;
-        cur = pop();
-      }
-      if (!__any_sync(__activemask(), leaf == kNone)) break;
+    bool hit[4];
+    float tn[4];
+    uint32_t ref[4];
+    quad_test(s.quads + cur, qr, tmin, bt * 1.000001f + 1e-30f, hit, tn, ref);
+    uint32_t leaves = 0u;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const bool leaf = hit[k] && (ref[k] & kLeafBit);
+      if (leaf) leaves |= 1u << k;
+      tn[k] = hit[k] && !leaf ? tn[k] : INFINITY;
     }
-    // the pending leaf, and any leaf reached right after it
-    while (leaf != kNone) {
-      if (it++ >= max_iter) {
-        errs += 1;
-        cur = kNone;
-        break;
-      }
+    while (leaves) {  // one code path, so that the lanes of the warp test their leaves together
+      const uint32_t k = (uint32_t)__ffs(leaves) - 1u;
+      leaves &= leaves - 1u;
+      const uint32_t lo = (k & 1u) ? ref[1] : ref[0], hi = (k & 1u) ? ref[3] : ref[2];
+      const uint32_t leaf = (k & 2u) ? hi : lo;
       if (!kChecked || leaf_in_range(s, leaf)) test_leaf(s, leaf, r, tnear, bt, bid, bref);
       else errs += 1;
-      leaf = kNone;
-      if (cur != kNone && (cur & kLeafBit)) {
-        leaf = cur;
-        cur = pop();
-      }
+    }
+    const bool s01 = tn[1] < tn[0], s23 = tn[3] < tn[2];
+    const float n01 = fminf(tn[0], tn[1]), x01 = fmaxf(tn[0], tn[1]);
+    const float n23 = fminf(tn[2], tn[3]), x23 = fmaxf(tn[2], tn[3]);
+    const uint32_t rn01 = s01 ? ref[1] : ref[0], rx01 = s01 ? ref[0] : ref[1];
+    const uint32_t rn23 = s23 ? ref[3] : ref[2], rx23 = s23 ? ref[2] : ref[3];
+    const bool swap = n23 < n01;
+    if (sp + 3 > STACK && sp + (x01 < INFINITY) + (x23 < INFINITY) + (fmaxf(n01, n23) < INFINITY) > STACK) {
+      errs += 1;
+      break;
+    }
+    if ((swap ? x01 : x23) < INFINITY) stack(sp++) = swap ? rx01 : rx23;
+    if ((swap ? n01 : n23) < INFINITY) stack(sp++) = swap ? rn01 : rn23;
+    if ((swap ? x23 : x01) < INFINITY) stack(sp++) = swap ? rx23 : rx01;
+    cur = swap ? rn23 : rn01;
+    if (!(fminf(n01, n23) < INFINITY)) {
+      if (sp == 0) break;
+      cur = stack(--sp);
     }
   }
   return bid != INT_MAX;
@@ -573,6 +584,14 @@ __device__ __forceinline__ double warp_sum_d(double v) {
   return v;
 }
 
+// Threads per SM that the register target leaves room for.  Forward: 1024 (64
+// registers, nothing spilled); 1152 and 896 measured 2.36 and 2.22 against
+// 2.20 ms on the 98 k-disc trench (1e6 rays), 27.1 and 29.7 against 26.5 ms on
+// 4.19 M discs.  The global adjoint: 768 (80 registers; at 64 it spills 138 B):
+// 1e6 rays into the hole 14.8 -> 13.8 ms, trench 2.66 -> 2.51; the field adjoint
+// loses more by the missing warps (4.19 M discs 7.96 -> 9.12 ms) and keeps 1024.
+constexpr int resident_threads(int mode) { return mode == kModeAdjGlobal ? 768 : 1024; }
+
 // kModeForward traces and deposits.  The adjoint modes replay the same paths
 // and accumulate derivatives of L = sum_i g_i S1_i instead.  G_k = the sum of g
 // over the primitives that received deposit k, v_k = w_k s its weight,
@@ -598,15 +617,13 @@ __device__ __forceinline__ double warp_sum_d(double v) {
 // Batched = true: lanes take global ray ids over the concatenated ray ranges
 // of `njobs` jobs (prefix[j] = first global id of job j) and trace each with
 // its job's parameters (scene, configuration, accumulators); the counters and
-// the abort flag are the batch's (p0).  TPB threads per block and 1024 / TPB
-// resident blocks per SM as the register target (64 registers per thread);
-// forward traces with 128 threads target 9 blocks (56 registers, a few spilled:
-// the extra warps hide more latency than the spills cost).
+// the abort flag are the batch's (p0).  TPB threads per block and
+// resident_threads(M) / TPB resident blocks per SM as the register target.
 // SHSTACK = true: the traversal stacks of the block live in shared memory
 // (STACK x TPB entries, at most 16 KB).  WIDE = true: closest hits over the
 // wide tree where a scene view carries one (see closest_hit).
-template <int M, bool Batched, int TPB, int STACK, bool POSTPONE = false, bool SHSTACK = false, bool WIDE = false>
-__global__ void __launch_bounds__(TPB, (M == kModeForward && TPB == 128 ? 1152 : 1024) / TPB)
+template <int M, bool Batched, int TPB, int STACK, bool SHSTACK = false, bool WIDE = false>
+__global__ void __launch_bounds__(TPB, resident_threads(M) / TPB)
     trace_paths_kernel(const __grid_constant__ TraceParams p0, const TraceParams* __restrict__ jobs,
                        const uint64_t* __restrict__ prefix, int njobs) {
   constexpr bool kAdj = M == kModeAdjGlobal || M == kModeAdjField;
@@ -745,7 +762,7 @@ __global__ void __launch_bounds__(TPB, (M == kModeForward && TPB == 128 ? 1152 :
     float th, tb = 0.0f;
     int hid;
     uint32_t href;
-    const bool hit = closest_hit<STACK, POSTPONE, kSst, WIDE>(pp->s, o, d, pp->tnear, th, hid, href, c_err, sstk);
+    const bool hit = closest_hit<STACK, kSst, WIDE>(pp->s, o, d, pp->tnear, th, hid, href, c_err, sstk);
     const int axis = boundary_exit(*pp, o, d, tb);
     if (kChecked && hit && (unsigned)hid >= (unsigned)(pp->s.nd + pp->s.nt)) {
       c_err += 1;
@@ -914,22 +931,19 @@ using PathKernel = void (*)(const TraceParams, const TraceParams*, const uint64_
 // The instantiation of trace_paths_kernel with its stack in shared memory
 // when `shared` asks for it and it fits 16 KB per block (8 blocks then leave
 // half of the SM's L1/shared capacity to L1), else in local memory; with the
-// wide traversal compiled in when `wide` (postponed leaf tests use the binary
-// tree only).
-template <int M, bool Batched, int TPB, int STACK, bool POSTPONE, bool WIDE>
+// wide traversal compiled in when `wide`.
+template <int M, bool Batched, int TPB, int STACK, bool WIDE>
 PathKernel kernel_for_width(bool shared) {
   if constexpr (STACK * TPB * 4 <= 16384) {
-    if (shared) return trace_paths_kernel<M, Batched, TPB, STACK, POSTPONE, true, WIDE>;
+    if (shared) return trace_paths_kernel<M, Batched, TPB, STACK, true, WIDE>;
   }
-  return trace_paths_kernel<M, Batched, TPB, STACK, POSTPONE, false, WIDE>;
+  return trace_paths_kernel<M, Batched, TPB, STACK, false, WIDE>;
 }
 
-template <int M, bool Batched, int TPB, int STACK, bool POSTPONE>
+template <int M, bool Batched, int TPB, int STACK>
 PathKernel kernel_for(bool shared, bool wide) {
-  if constexpr (!POSTPONE) {
-    if (wide) return kernel_for_width<M, Batched, TPB, STACK, false, true>(shared);
-  }
-  return kernel_for_width<M, Batched, TPB, STACK, POSTPONE, false>(shared);
+  return wide ? kernel_for_width<M, Batched, TPB, STACK, true>(shared)
+              : kernel_for_width<M, Batched, TPB, STACK, false>(shared);
 }
 
 }  // namespace

@@ -18,7 +18,7 @@ __global__ void closest_hit_kernel(const SceneView s, const float* __restrict__ 
   int id;
   uint32_t ref;
   unsigned long long e = 0;
-  if (closest_hit<256, false>(s, mk3(r[0], r[1], r[2]), mk3(r[3], r[4], r[5]), tnear, t, id, ref, e)) {
+  if (closest_hit<256>(s, mk3(r[0], r[1], r[2]), mk3(r[3], r[4], r[5]), tnear, t, id, ref, e)) {
     prim[i] = id;
     tout[i] = t;
   } else {
@@ -28,49 +28,44 @@ __global__ void closest_hit_kernel(const SceneView s, const float* __restrict__ 
   if (e) atomicAdd(errors, e);
 }
 
-template <int TPB, bool POSTPONE>
-PathKernel forward_kernel(int stack, bool shared, bool wide) {
-  if (stack <= 32) return kernel_for<kModeForward, false, TPB, 32, POSTPONE>(shared, wide);
-  if (stack <= 64) return kernel_for<kModeForward, false, TPB, 64, POSTPONE>(shared, wide);
-  return kernel_for<kModeForward, false, TPB, 256, POSTPONE>(shared, wide);
-}
-
 template <int TPB>
-PathKernel forward_kernel(int stack, bool postpone, bool shared, bool wide) {
-  return postpone ? forward_kernel<TPB, true>(stack, shared, wide) : forward_kernel<TPB, false>(stack, shared, wide);
+PathKernel forward_kernel(int stack, bool shared, bool wide) {
+  if (stack <= 32) return kernel_for<kModeForward, false, TPB, 32>(shared, wide);
+  if (stack <= 64) return kernel_for<kModeForward, false, TPB, 64>(shared, wide);
+  return kernel_for<kModeForward, false, TPB, 256>(shared, wide);
 }
 
 // The adjoint replays run with 128 threads and a 64- or 256-entry stack.
-PathKernel pick_kernel(int mode, int tpb, int stack, bool postpone, bool shared, bool wide, int& tpb_out) {
+PathKernel pick_kernel(int mode, int tpb, int stack, bool shared, bool wide, int& tpb_out) {
   if (mode == kModeAdjGlobal) {
     tpb_out = 128;
-    if (stack <= 64) return kernel_for<kModeAdjGlobal, false, 128, 64, false>(shared, wide);
-    return wide ? trace_paths_kernel<kModeAdjGlobal, false, 128, 256, false, false, true>
+    if (stack <= 64) return kernel_for<kModeAdjGlobal, false, 128, 64>(shared, wide);
+    return wide ? trace_paths_kernel<kModeAdjGlobal, false, 128, 256, false, true>
                 : trace_paths_kernel<kModeAdjGlobal, false, 128, 256>;
   }
   if (mode == kModeAdjField) {
     tpb_out = 128;
-    if (stack <= 64) return kernel_for<kModeAdjField, false, 128, 64, false>(shared, wide);
-    return wide ? trace_paths_kernel<kModeAdjField, false, 128, 256, false, false, true>
+    if (stack <= 64) return kernel_for<kModeAdjField, false, 128, 64>(shared, wide);
+    return wide ? trace_paths_kernel<kModeAdjField, false, 128, 256, false, true>
                 : trace_paths_kernel<kModeAdjField, false, 128, 256>;
   }
   if (mode == kModeLogged) {  // a debugging trace: one configuration, both trees
     tpb_out = 128;
-    return trace_paths_kernel<kModeLogged, false, 128, 256, false, false, true>;
+    return trace_paths_kernel<kModeLogged, false, 128, 256, false, true>;
   }
   if (mode == kModeWindow) {
     tpb_out = 128;
     if (stack <= 64)
-      return wide ? trace_paths_kernel<kModeWindow, false, 128, 64, false, false, true>
+      return wide ? trace_paths_kernel<kModeWindow, false, 128, 64, false, true>
                   : trace_paths_kernel<kModeWindow, false, 128, 64>;
-    return wide ? trace_paths_kernel<kModeWindow, false, 128, 256, false, false, true>
+    return wide ? trace_paths_kernel<kModeWindow, false, 128, 256, false, true>
                 : trace_paths_kernel<kModeWindow, false, 128, 256>;
   }
   tpb_out = tpb;
-  if (tpb == 64) return forward_kernel<64>(stack, postpone, shared, wide);
-  if (tpb == 256) return forward_kernel<256>(stack, postpone, shared, wide);
+  if (tpb == 64) return forward_kernel<64>(stack, shared, wide);
+  if (tpb == 256) return forward_kernel<256>(stack, shared, wide);
   tpb_out = 128;
-  return forward_kernel<128>(stack, postpone, shared, wide);
+  return forward_kernel<128>(stack, shared, wide);
 }
 
 }  // namespace
@@ -151,7 +146,7 @@ bool use_wide(const rtg_context* ctx) {
 }
 
 int traversal_depth(const rtg_context* ctx) {
-  return use_wide(ctx) ? std::max(ctx->g.depth, ctx->g.wide_stack) : ctx->g.depth;
+  return use_wide(ctx) ? ctx->g.wide_stack : ctx->g.quad_stack;
 }
 
 SceneView scene_view(rtg_context* ctx) {
@@ -165,6 +160,7 @@ SceneView scene_view(rtg_context* ctx) {
   s.tri = g.tri.p;
   s.nt = (int32_t)g.nt;
   s.nodes = g.nodes.p;
+  s.quads = g.quads.p;
   s.root = g.root;
   s.nb_ptr = g.nd > 0 ? g.nb_ptr.p : nullptr;
   s.nb_slot = g.nb_slot.p;
@@ -177,7 +173,6 @@ SceneView scene_view(rtg_context* ctx) {
 
 int launch_trace(rtg_context* ctx, const TraceParams& p_in, cudaStream_t st, int mode) {
   const rtg_launch_config& lc = ctx->lc;
-  const int stack = stack_for(lc.stack_depth, traversal_depth(ctx));
   TraceParams p = p_in;
   p.packet = lc.packet;
   const uint64_t nrays = p.ray_end - p.ray_begin;
@@ -185,6 +180,9 @@ int launch_trace(rtg_context* ctx, const TraceParams& p_in, cudaStream_t st, int
   // so has a trace that fills the segment log
   if (mode == kModeForward && p.window) mode = kModeWindow;
   if (mode == kModeForward && p.log.rec) mode = kModeLogged;
+  // the window's interval queries walk the binary tree
+  const int need = mode == kModeWindow ? std::max(ctx->g.depth, traversal_depth(ctx)) : traversal_depth(ctx);
+  const int stack = stack_for(lc.stack_depth, need);
   if (mode == kModeForward && lc.scheduling == RTG_SCHED_WAVEFRONT) {
     // a job table of one entry
     Wavefront& wf = ctx->wf;
@@ -197,15 +195,14 @@ int launch_trace(rtg_context* ctx, const TraceParams& p_in, cudaStream_t st, int
     return launch_wavefront(ctx, p, wf.one_job.p, wf.one_prefix.p, 1, nrays, st, lc, traversal_depth(ctx));
   }
   int tpb = 128, sms = 0, per_sm = 0;
-  PathKernel kern = pick_kernel(mode, lc.threads_per_block, stack, lc.leaf_tests == RTG_LEAF_POSTPONED,
-                                shared_stack(ctx, lc), p.s.wnodes != nullptr, tpb);
+  PathKernel kern = pick_kernel(mode, lc.threads_per_block, stack, shared_stack(ctx, lc), p.s.wnodes != nullptr, tpb);
   p.plain = (mode == kModeForward || mode == kModeWindow) && lc.scheduling == RTG_SCHED_PLAIN ? 1 : 0;
   RTG_CUDA(ctx, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
   RTG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, tpb, 0));
   if (per_sm < 1) per_sm = 1;
   uint64_t blocks = (uint64_t)sms * per_sm;
-  const uint64_t need = (nrays + tpb - 1) / tpb;
-  if (need < blocks || p.plain) blocks = need > 0 ? need : 1;
+  const uint64_t full = (nrays + tpb - 1) / tpb;
+  if (full < blocks || p.plain) blocks = full > 0 ? full : 1;
   if (blocks > 0x7FFFFFFFull) return set_error(ctx, RTG_ERR_INVALID_ARGUMENT, "too many rays for a plain launch");
   kern<<<(unsigned)blocks, tpb, 0, st>>>(p, nullptr, nullptr, 0);
   RTG_CUDA(ctx, cudaGetLastError());

@@ -6,16 +6,11 @@ namespace rtg {
 
 namespace {
 
-template <int TPB, bool POSTPONE>
-PathKernel batched_kernel(int stack, bool shared, bool wide) {
-  if (stack <= 32) return kernel_for<kModeForward, true, TPB, 32, POSTPONE>(shared, wide);
-  if (stack <= 64) return kernel_for<kModeForward, true, TPB, 64, POSTPONE>(shared, wide);
-  return kernel_for<kModeForward, true, TPB, 256, POSTPONE>(shared, wide);
-}
-
 template <int TPB>
-PathKernel batched_kernel(int stack, bool postpone, bool shared, bool wide) {
-  return postpone ? batched_kernel<TPB, true>(stack, shared, wide) : batched_kernel<TPB, false>(stack, shared, wide);
+PathKernel batched_kernel(int stack, bool shared, bool wide) {
+  if (stack <= 32) return kernel_for<kModeForward, true, TPB, 32>(shared, wide);
+  if (stack <= 64) return kernel_for<kModeForward, true, TPB, 64>(shared, wide);
+  return kernel_for<kModeForward, true, TPB, 256>(shared, wide);
 }
 
 }  // namespace
@@ -30,11 +25,10 @@ int launch_trace_batched(rtg_context* ctx, const TraceParams& p0_in, const Trace
   p0.packet = lc.packet;
   p0.plain = lc.scheduling == RTG_SCHED_PLAIN ? 1 : 0;
   int tpb = lc.threads_per_block, sms = 0, per_sm = 0;
-  const bool pp = lc.leaf_tests == RTG_LEAF_POSTPONED;
   const bool sh = lc.stack_memory == RTG_STACK_SHARED;  // AUTO: local (the jobs' trees differ in size)
-  PathKernel kern = tpb == 64    ? batched_kernel<64>(stack, pp, sh, wide)
-                    : tpb == 256 ? batched_kernel<256>(stack, pp, sh, wide)
-                                 : batched_kernel<128>(stack, pp, sh, wide);
+  PathKernel kern = tpb == 64    ? batched_kernel<64>(stack, sh, wide)
+                    : tpb == 256 ? batched_kernel<256>(stack, sh, wide)
+                                 : batched_kernel<128>(stack, sh, wide);
   if (tpb != 64 && tpb != 256) tpb = 128;
   RTG_CUDA(ctx, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
   RTG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, tpb, 0));

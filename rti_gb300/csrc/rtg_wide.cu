@@ -227,7 +227,7 @@ __global__ void wide_init_kernel(uint32_t* w2b, uint32_t* need, unsigned int* ct
 }  // namespace
 
 bool wants_wide(const rtg_context* ctx) {
-  return ctx->node_width == RTG_NODES_WIDE || (ctx->node_width == RTG_NODES_AUTO && outgrows_l2(ctx));
+  return ctx->node_width == RTG_NODES_WIDE;
 }
 
 int ensure_wide(rtg_context* ctx) {

@@ -220,8 +220,8 @@ class Engine:
         return w.value == L.RTG_NODES_WIDE
 
     def set_node_width(self, width: int):
-        """L.RTG_NODES_AUTO (default: wide when the tree outgrows L2), L.RTG_NODES_BINARY
-        or L.RTG_NODES_WIDE (the compressed 8-wide tree); results do not depend on it."""
+        """L.RTG_NODES_AUTO (default) and L.RTG_NODES_BINARY: float boxes, four a visit;
+        L.RTG_NODES_WIDE: the compressed 8-wide tree; results do not depend on it."""
         self._check(self._L.rtg_set_node_width(self._h, int(width)))
 
     @property
