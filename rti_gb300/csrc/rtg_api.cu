@@ -110,23 +110,48 @@ __device__ __forceinline__ void atomic_max_f(float* a, float v) {
   else atomicMin((unsigned int*)a, __float_as_uint(v));
 }
 
-// Warp minima/maxima of (x, y, z), then one atomic per warp.
-__device__ __forceinline__ void bounds_add(UploadCheck* c, float x, float y, float z, bool valid) {
-  float l[3] = {valid ? x : FLT_MAX, valid ? y : FLT_MAX, valid ? z : FLT_MAX};
-  float h[3] = {valid ? x : -FLT_MAX, valid ? y : -FLT_MAX, valid ? z : -FLT_MAX};
+// Bounds that a thread has seen, reduced over the block: one atomic per block
+// and bound (one per warp and 32 elements kept the L2 atomics busy).
+struct Bounds {
+  float l[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, h[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX}, r = 0.0f;
+  __device__ __forceinline__ void add(float x, float y, float z) {
+    l[0] = fminf(l[0], x);
+    l[1] = fminf(l[1], y);
+    l[2] = fminf(l[2], z);
+    h[0] = fmaxf(h[0], x);
+    h[1] = fmaxf(h[1], y);
+    h[2] = fmaxf(h[2], z);
+  }
+  __device__ void reduce(UploadCheck* c) {  // all threads of the block call it
+    __shared__ float red[8][7];             // 256 threads
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
+    for (int o = 16; o > 0; o >>= 1) {
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      l[a] = fminf(l[a], __shfl_xor_sync(0xFFFFFFFFu, l[a], o));
-      h[a] = fmaxf(h[a], __shfl_xor_sync(0xFFFFFFFFu, h[a], o));
+      for (int a = 0; a < 3; ++a) {
+        l[a] = fminf(l[a], __shfl_xor_sync(0xFFFFFFFFu, l[a], o));
+        h[a] = fmaxf(h[a], __shfl_xor_sync(0xFFFFFFFFu, h[a], o));
+      }
+      r = fmaxf(r, __shfl_xor_sync(0xFFFFFFFFu, r, o));
     }
-  if ((threadIdx.x & 31) == 0)
-    for (int a = 0; a < 3; ++a) {
-      atomic_min_f(&c->lo[a], l[a]);
-      atomic_max_f(&c->hi[a], h[a]);
+    if (lane == 0) {
+      for (int a = 0; a < 3; ++a) {
+        red[warp][a] = l[a];
+        red[warp][3 + a] = h[a];
+      }
+      red[warp][6] = r;
     }
-}
+    __syncthreads();
+    const int k = threadIdx.x;
+    if (k < 7) {
+      float v = red[0][k];
+      for (int w = 1; w < 8; ++w) v = k < 3 ? fminf(v, red[w][k]) : fmaxf(v, red[w][k]);
+      if (k < 3) atomic_min_f(&c->lo[k], v);
+      else if (k < 6) atomic_max_f(&c->hi[k - 3], v);
+      else atomic_max_f(&c->rmax, v);
+    }
+  }
+};
 
 __global__ void check_init_kernel(UploadCheck* c) {
   for (int a = 0; a < 3; ++a) {
@@ -143,38 +168,35 @@ __device__ __forceinline__ bool finite3_d(float x, float y, float z) {
 }
 
 // Disc i: finite centre, normal and radius, radius > 0, unit normal (within
-// 1e-3); writes (centre, r) and (normal, 0).  Grid-stride; whole warps.
-__global__ void disc_check_kernel(const float* __restrict__ pts, const float* __restrict__ nrm,
-                                  const float* __restrict__ rad, int64_t n, float4* __restrict__ cr,
-                                  float4* __restrict__ nn, UploadCheck* c) {
+// 1e-3); writes (centre, r) and (normal, 0).
+__global__ void __launch_bounds__(256) disc_check_kernel(const float* __restrict__ pts, const float* __restrict__ nrm,
+                                                          const float* __restrict__ rad, int64_t n,
+                                                          float4* __restrict__ cr, float4* __restrict__ nn,
+                                                          UploadCheck* c) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n; base += stride) {
-    const int64_t i = base + threadIdx.x;
-    const bool in = i < n;
-    float p[3] = {0, 0, 0}, q[3] = {0, 0, 1}, r = 1.0f;
-    if (in)
-      for (int a = 0; a < 3; ++a) {
-        p[a] = pts[3 * i + a];
-        q[a] = nrm[3 * i + a];
-      }
-    if (in) r = rad[i];
+  Bounds b;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+    float p[3], q[3];
+    for (int a = 0; a < 3; ++a) {
+      p[a] = pts[3 * i + a];
+      q[a] = nrm[3 * i + a];
+    }
+    const float r = rad[i];
     bool ok = finite3_d(p[0], p[1], p[2]) && finite3_d(q[0], q[1], q[2]) && isfinite(r) && r > 0.0f;
     if (ok) {
       const float l2 = q[0] * q[0] + q[1] * q[1] + q[2] * q[2];
       ok = fabsf(sqrtf(l2) - 1.0f) <= 1e-3f;
     }
-    if (in && !ok) atomicMin(&c->bad, (unsigned long long)i);
-    if (in) {
-      cr[i] = make_float4(p[0], p[1], p[2], r);
-      nn[i] = make_float4(q[0], q[1], q[2], 0.0f);
+    cr[i] = make_float4(p[0], p[1], p[2], r);
+    nn[i] = make_float4(q[0], q[1], q[2], 0.0f);
+    if (ok) {
+      b.add(p[0], p[1], p[2]);
+      b.r = fmaxf(b.r, r);
+    } else {
+      atomicMin(&c->bad, (unsigned long long)i);
     }
-    const bool v = in && ok;
-    bounds_add(c, p[0], p[1], p[2], v);
-    float rm = v ? r : 0.0f;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) rm = fmaxf(rm, __shfl_xor_sync(0xFFFFFFFFu, rm, o));
-    if ((threadIdx.x & 31) == 0) atomic_max_f(&c->rmax, rm);
   }
+  b.reduce(c);
 }
 
 // Vertex i: finite; writes (x, y, z, 0).
@@ -188,27 +210,41 @@ __global__ void vertex_check_kernel(const float* __restrict__ v, int64_t nv, flo
   }
 }
 
-// Triangle t: its three indices below nv; bounds over the vertices it uses.
-__global__ void triangle_check_kernel(const uint32_t* __restrict__ idx, int64_t nt, int64_t nv,
-                                      const float4* __restrict__ vert, UploadCheck* c) {
+// The same with the bounds of all vertices.
+__global__ void __launch_bounds__(256) vertex_bounds_kernel(const float* __restrict__ v, int64_t nv,
+                                                             float4* __restrict__ out, UploadCheck* c) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < nt; base += stride) {
-    const int64_t t = base + threadIdx.x;
-    const bool in = t < nt;
-    for (int k = 0; k < 3; ++k) {
-      const uint32_t q = in ? idx[3 * t + k] : 0u;
-      const bool ok = in && (int64_t)q < nv;
-      if (in && !ok) atomicMin(&c->bad_tri, (unsigned long long)t);
-      float4 p = make_float4(0, 0, 0, 0);
-      if (ok) p = vert[q];
-      bounds_add(c, p.x, p.y, p.z, ok);
-    }
+  Bounds b;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += stride) {
+    const float x = v[3 * i], y = v[3 * i + 1], z = v[3 * i + 2];
+    if (finite3_d(x, y, z)) b.add(x, y, z);
+    else atomicMin(&c->bad, (unsigned long long)i);
+    out[i] = make_float4(x, y, z, 0.0f);
   }
+  b.reduce(c);
+}
+
+// Triangle t: its three indices below nv; bounds over the vertices it uses.
+__global__ void __launch_bounds__(256) triangle_check_kernel(const uint32_t* __restrict__ idx, int64_t nt, int64_t nv,
+                                                              const float4* __restrict__ vert, UploadCheck* c) {
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  Bounds b;
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < nt; t += stride)
+    for (int k = 0; k < 3; ++k) {
+      const uint32_t q = idx[3 * t + k];
+      if ((int64_t)q < nv) {
+        const float4 p = vert[q];
+        b.add(p.x, p.y, p.z);
+      } else {
+        atomicMin(&c->bad_tri, (unsigned long long)t);
+      }
+    }
+  b.reduce(c);
 }
 
 unsigned grid_for(int64_t n) {
   const int64_t b = (n + 255) / 256;
-  return (unsigned)std::max<int64_t>(1, std::min<int64_t>(b, 4096));
+  return (unsigned)std::max<int64_t>(1, std::min<int64_t>(b, 152 * 4));
 }
 
 // An upload checked on the device and not yet part of the context.
@@ -318,6 +354,33 @@ int stage_triangles(rtg_context* ctx, const float* vertices, const uint32_t* ind
   else if (rc == RTG_OK && sg.ht.bad_tri != ~0ull)
     rc = set_error(ctx, RTG_ERR_INVALID_ARGUMENT,
                    "triangle " + std::to_string(sg.ht.bad_tri) + ": vertex index out of range");
+  return rc;
+}
+
+// Copies nv vertices to the device and checks them there (one synchronisation).
+int stage_vertices(rtg_context* ctx, const float* vertices, int64_t nv, Staged& sg) {
+  cudaStream_t st = ctx->stream;
+  sg.nv = nv;
+  check_reset(sg.ht);
+  DBuf<float> raw;
+  DBuf<UploadCheck> chk;
+  int rc = talloc(ctx, chk, 1, st, "vertex update");
+  if (rc == RTG_OK) rc = talloc(ctx, raw, (size_t)(3 * nv), st, "vertex update");
+  if (rc == RTG_OK) rc = talloc(ctx, sg.v4, (size_t)nv, st, "vertex update");
+  if (rc == RTG_OK) {
+    cudaError_t e = cudaMemcpyAsync(raw.p, vertices, 3 * nv * sizeof(float), cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) {
+      check_init_kernel<<<1, 1, 0, st>>>(chk.p);
+      vertex_bounds_kernel<<<grid_for(nv), 256, 0, st>>>(raw.p, nv, sg.v4.p, chk.p);
+      e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&sg.ht, chk.p, sizeof sg.ht, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) rc = check_cuda(ctx, e, "vertex update");
+  }
+  tfree(raw, st);
+  tfree(chk, st);
+  if (rc == RTG_OK && sg.ht.bad != ~0ull) rc = set_error(ctx, RTG_ERR_INVALID_ARGUMENT, "vertex is not finite");
   return rc;
 }
 
@@ -440,10 +503,29 @@ int prepare_trace(rtg_context* ctx, uint64_t ray_begin, uint64_t ray_end, uint64
   return prepare_trace_with(ctx, ctx->cfg, ctx->box_lo, ctx->box_hi, ray_begin, ray_end, seed, p);
 }
 
-int rebuild_all(rtg_context* ctx) {
-  RTG_TRY(build_lbvh(ctx));
-  RTG_TRY(build_neighbors(ctx));
+// Scratch that building a surface takes: the staged arrays, the sort, the
+// neighbour grid and the tree's temporaries (a clustering's buffers more).
+size_t build_scratch(const rtg_context* ctx, int64_t nd, int64_t nv, int64_t nt) {
+  const int64_t np = nd + nt;
+  return (size_t)(160 * nd + 28 * nv + 12 * nt + 96 * np + (ctx->g.builder == kBuilderPloc ? 96 * np : 0)) + 262144;
+}
+
+// The tree (built anew, or refitted in place) and the neighbour lists; waits
+// until they are complete.
+int rebuild(rtg_context* ctx, bool refit) {
+  NeighborWork w;
+  int rc = count_neighbors(ctx, w);
+  if (rc == RTG_OK) rc = refit ? refit_lbvh(ctx) : build_lbvh(ctx);
+  if (rc == RTG_OK) rc = fill_neighbors(ctx, w);
+  release_neighbors(w, ctx->stream);
+  const cudaError_t e = cudaStreamSynchronize(ctx->stream);
+  if (rc == RTG_OK && e != cudaSuccess) rc = check_cuda(ctx, e, "surface build");
+  return rc;
+}
+
+int rebuild_all(rtg_context* ctx, bool refit) {
   RTG_TRY(alloc_results(ctx));
+  RTG_TRY(rebuild(ctx, refit));
   resolve_box(ctx);
   return RTG_OK;
 }
@@ -534,6 +616,7 @@ int rtg_destroy(rtg_context* ctx) {
   dfree(g.refit_flags); dfree(g.nb_ptr); dfree(g.nb_idx); dfree(g.nb_slot); dfree(g.disc_slot);
   dfree(ctx->sticking_field); dfree(ctx->acc); dfree(ctx->cnt); dfree(ctx->areas); dfree(ctx->est);
   dfree(ctx->stat_tmp);
+  dfree(ctx->scratch);
   dfree(g.wnodes);
   dfree(ctx->seglog);
   dfree(ctx->seglog_count);
@@ -557,6 +640,8 @@ int rtg_upload_mixed(rtg_context* ctx, const float* points, const float* normals
   if (!ctx) return RTG_ERR_INVALID_ARGUMENT;
   NvtxRange range("rtg upload + LBVH build");
   RTG_TRY(use_device(ctx));
+  ScratchScope scratch(ctx, build_scratch(ctx, std::max<int64_t>(nd, 0), std::max<int64_t>(nv, 0),
+                                          std::max<int64_t>(nt, 0)));
   // both halves are checked before either replaces the context's surface
   Staged sg;
   int rc = stage_discs(ctx, points, normals, radii, nd, sg);
@@ -570,7 +655,7 @@ int rtg_upload_mixed(rtg_context* ctx, const float* points, const float* normals
   release(sg, ctx->stream);
   if (committing) {
     dfree(ctx->sticking_field);
-    if (rc == RTG_OK) rc = rebuild_all(ctx);
+    if (rc == RTG_OK) rc = rebuild_all(ctx, false);
     if (rc != RTG_OK) drop_surface(ctx);
   }
   return rc;
@@ -590,6 +675,7 @@ int rtg_update_discs(rtg_context* ctx, const float* points, const float* normals
   RTG_TRY(use_device(ctx));
   if (n != ctx->g.nd)
     return set_error(ctx, RTG_ERR_INVALID_ARGUMENT, "update_discs: the disc count must not change");
+  ScratchScope scratch(ctx, build_scratch(ctx, ctx->g.nd, 0, ctx->g.nt));
   Staged sg;
   int rc = stage_discs(ctx, points, normals, radii, n, sg);
   const bool committing = rc == RTG_OK;
@@ -599,15 +685,9 @@ int rtg_update_discs(rtg_context* ctx, const float* points, const float* normals
   }
   release(sg, ctx->stream);
   if (!committing) return rc;
-  if (rc == RTG_OK) rc = refit_lbvh(ctx);
-  if (rc == RTG_OK) rc = build_neighbors(ctx);
-  if (rc == RTG_OK) rc = alloc_results(ctx);
-  if (rc != RTG_OK) {
-    drop_surface(ctx);
-    return rc;
-  }
-  resolve_box(ctx);
-  return RTG_OK;
+  if (rc == RTG_OK) rc = rebuild_all(ctx, true);
+  if (rc != RTG_OK) drop_surface(ctx);
+  return rc;
 }
 
 static int rtg_update_vertices_body(rtg_context* ctx, const float* vertices, int64_t nv);
@@ -622,31 +702,24 @@ static int rtg_update_vertices_body(rtg_context* ctx, const float* vertices, int
   if (g.nt == 0 || nv != g.nv || !vertices)
     return set_error(ctx, RTG_ERR_INVALID_ARGUMENT, "update_vertices: vertex count must match the upload");
   RTG_TRY(use_device(ctx));
-  std::vector<float4> v((size_t)nv);
-  float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-  for (int64_t i = 0; i < nv; ++i) {
-    if (!finite3(vertices + 3 * i)) return set_error(ctx, RTG_ERR_INVALID_ARGUMENT, "vertex is not finite");
-    v[(size_t)i] = make_float4(vertices[3 * i], vertices[3 * i + 1], vertices[3 * i + 2], 0.0f);
-    for (int a = 0; a < 3; ++a) {
-      lo[a] = std::min(lo[a], vertices[3 * i + a]);
-      hi[a] = std::max(hi[a], vertices[3 * i + a]);
-    }
-  }
-  for (int a = 0; a < 3; ++a) {
-    g.tri_min[a] = lo[a];
-    g.tri_max[a] = hi[a];
-  }
-  ++ctx->version;
-  int rc = check_cuda(ctx, cudaMemcpyAsync(g.tri_v.p, v.data(), nv * sizeof(float4), cudaMemcpyHostToDevice,
-                                           ctx->stream), "vertex update");
-  if (rc == RTG_OK) rc = refit_lbvh(ctx);
-  if (rc == RTG_OK) rc = alloc_results(ctx);
+  ScratchScope scratch(ctx, build_scratch(ctx, g.nd, 0, g.nt));
+  Staged sg;
+  int rc = stage_vertices(ctx, vertices, nv, sg);
   if (rc != RTG_OK) {
-    drop_surface(ctx);
+    release(sg, ctx->stream);
     return rc;
   }
-  resolve_box(ctx);
-  return RTG_OK;
+  for (int a = 0; a < 3; ++a) {
+    g.tri_min[a] = sg.ht.lo[a];
+    g.tri_max[a] = sg.ht.hi[a];
+  }
+  ++ctx->version;
+  rc = check_cuda(ctx, cudaMemcpyAsync(g.tri_v.p, sg.v4.p, nv * sizeof(float4), cudaMemcpyDeviceToDevice, ctx->stream),
+                  "vertex update");
+  release(sg, ctx->stream);
+  if (rc == RTG_OK) rc = rebuild_all(ctx, true);
+  if (rc != RTG_OK) drop_surface(ctx);
+  return rc;
 }
 
 int rtg_set_config(rtg_context* ctx, const rtg_config* cfg) {
@@ -762,11 +835,11 @@ int rtg_set_tree_builder(rtg_context* ctx, int32_t builder) {
   RTG_TRY(use_device(ctx));
   const int32_t keep = ctx->g.builder;
   ctx->g.builder = builder;
+  ScratchScope scratch(ctx, build_scratch(ctx, ctx->g.nd, 0, ctx->g.nt));
   if (ctx->g.nd + ctx->g.nt > 0 && ctx->g.nodes.p && builder != keep) {
     ++ctx->version;
     int rc = check_cuda(ctx, cudaStreamSynchronize(ctx->stream), "tree rebuild");
-    if (rc == RTG_OK) rc = build_lbvh(ctx);
-    if (rc == RTG_OK) rc = build_neighbors(ctx);  // neighbour columns are stored as slots of the new tree
+    if (rc == RTG_OK) rc = rebuild(ctx, false);  // neighbour columns are stored as slots of the new tree
     if (rc != RTG_OK) {
       drop_surface(ctx);
       return rc;

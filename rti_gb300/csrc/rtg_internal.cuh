@@ -17,10 +17,10 @@ namespace rtg {
 constexpr uint32_t kLeafBit = 0x80000000u;
 constexpr uint32_t kTriBit = 0x40000000u;
 constexpr uint32_t kSlotMask = 0x3FFFFFFFu;
-// deepest binary tree kept (the radix tree's depth is bounded by its 62 key
-// bits; a clustering deeper than this falls back to it): the largest traversal
-// stack holds 256 entries, and a quad's can exceed the binary one by 64
-constexpr int kMaxDepth = 192;
+// the largest traversal stack, and the deepest binary tree kept (the radix
+// tree's depth is bounded by its 62 key bits; a deeper clustering falls back to it)
+constexpr int kMaxStack = 256;
+constexpr int kMaxDepth = 256;
 
 // One internal node: the boxes of both children and their references (64 B).
 //   a = (c0.lo.x, c0.hi.x, c1.lo.x, c1.hi.x)
@@ -39,7 +39,7 @@ struct __align__(16) Node {
 //   xy[k] = (centre.x, centre.y, half.x, half.y) of child k
 //   z[j]  = (centre.z of 2j, of 2j + 1, half.z of 2j, of 2j + 1)
 //   ref   = the children's references; a missing child has half extents -1e30
-//           (a box that no ray meets)
+//           (a box that no ray meets) and a leaf reference
 // The half extents are rounded up and widened by 2^-20 of themselves and 2^-21
 // of the centre, which covers the rounding of the slab test (quad_test in
 // rtg_path.cuh) for rays that start near the box; the test's relative slack
@@ -48,7 +48,7 @@ struct __align__(128) QuadNode {
   float4 xy[4];
   float4 z[2];
   uint4 ref;
-  uint4 unused;
+  uint4 info;  // x: inner children
 };
 
 // One node of the compressed 8-wide tree the closest-hit query may traverse
@@ -167,6 +167,7 @@ template <typename T>
 struct DBuf {
   T* p = nullptr;
   size_t n = 0;
+  bool scratch = false;  // a piece of the context's scratch buffer (talloc)
 };
 
 struct Geometry {
@@ -234,7 +235,11 @@ struct rtg_context {
   rtg::DBuf<unsigned long long> cnt;
   rtg::DBuf<float> areas;
   rtg::DBuf<float> est;
-  rtg::DBuf<double> stat_tmp;
+  rtg::DBuf<double> stat_tmp;  // statistics: relative error | vov; estimates: the maximum | S1 per area
+  // temporaries of builds (ScratchScope)
+  rtg::DBuf<unsigned char> scratch;
+  size_t scratch_top = 0;
+  bool scratch_open = false;
   // segment log (rtg_set_segment_log)
   rtg::DBuf<rtg_segment> seglog;
   rtg::DBuf<unsigned long long> seglog_count;
@@ -278,7 +283,7 @@ struct NvtxRange {
 int exclusive_scan_u32(rtg_context* ctx, uint32_t* d_a, int64_t m, uint32_t* d_total, cudaStream_t st);
 int exclusive_scan_i64(rtg_context* ctx, int64_t* d_a, int64_t m, int64_t* d_total, cudaStream_t st);
 int radix_sort_pairs(rtg_context* ctx, uint32_t* d_keys, uint32_t* d_vals, uint32_t* d_tmp_keys,
-                     uint32_t* d_tmp_vals, int64_t n, int bits, cudaStream_t st);
+                     uint32_t* d_tmp_vals, int64_t n, int bits, unsigned long long* d_errors, cudaStream_t st);
 // lbvh.cu
 int build_lbvh(rtg_context* ctx);      // full build from the by-id primitive data
 int refit_lbvh(rtg_context* ctx);      // recompute boxes, keep topology
@@ -289,8 +294,18 @@ int build_wide(rtg_context* ctx, cudaStream_t st);
 bool wants_wide(const rtg_context* ctx);
 // collapses the wide tree if it is wanted and not current (synchronises)
 int ensure_wide(rtg_context* ctx);
-// surface.cu
-int build_neighbors(rtg_context* ctx);
+// surface.cu: the neighbour lists, their row lengths before the tree is built
+// and the rows after it
+struct NeighborWork {
+  DBuf<uint32_t> start, cell_id;
+  DBuf<uint2> cell_rank;
+  DBuf<float4> cell_disc;
+  float org[3] = {0, 0, 0}, inv_h = 0;
+  int dim[3] = {0, 0, 0};
+};
+int count_neighbors(rtg_context* ctx, NeighborWork& w);
+int fill_neighbors(rtg_context* ctx, NeighborWork& w);
+void release_neighbors(NeighborWork& w, cudaStream_t st);
 int compute_areas(rtg_context* ctx, cudaStream_t st, const float* box_lo, const float* box_hi);
 int finalize_estimates(rtg_context* ctx, cudaStream_t st);
 int compute_stats(rtg_context* ctx, cudaStream_t st, uint64_t total, double* d_rel, double* d_vov);
@@ -395,9 +410,41 @@ void dfree(DBuf<T>& b) {
   b.p = nullptr;
   b.n = 0;
 }
-// Temporaries of a build step: stream-ordered allocations from the device's
-// memory pool, released on the same stream without the device-wide
-// synchronisation of cudaFree.
+// Temporaries of a build, for a call that runs on the context's stream and
+// waits for it: inside a ScratchScope they are cut from the context's scratch
+// buffer, which the context keeps (the device's default pool gives its memory
+// back at every synchronisation, and mapping it anew took 0.2 ms of a 0.6 ms
+// upload); what does not fit, and calls outside a scope, take stream-ordered
+// allocations from that pool.
+constexpr size_t kScratchMax = (size_t)64 << 20;  // kept per context; a larger surface's build dwarfs the mapping
+struct ScratchScope {
+  rtg_context* ctx;
+  bool outer;
+  // bytes: what the call's temporaries are expected to take
+  ScratchScope(rtg_context* c, size_t bytes) : ctx(c), outer(!c->scratch_open) {
+    if (!outer) return;
+    ctx->scratch_top = 0;
+    if (bytes <= kScratchMax && bytes > ctx->scratch.n) {
+      dfree(ctx->scratch);
+      void* p = nullptr;
+      bytes = (bytes + bytes / 2 + 65535) / 65536 * 65536;  // some room for the next surface
+      if (bytes > kScratchMax) bytes = kScratchMax;
+      if (cudaMalloc(&p, bytes) == cudaSuccess) {
+        ctx->scratch.p = (unsigned char*)p;
+        ctx->scratch.n = bytes;
+      } else {
+        cudaGetLastError();  // the pool serves the temporaries, or reports that there is no room
+      }
+    }
+    ctx->scratch_open = true;
+  }
+  ~ScratchScope() {
+    if (outer) ctx->scratch_open = false;
+  }
+  ScratchScope(const ScratchScope&) = delete;
+  ScratchScope& operator=(const ScratchScope&) = delete;
+};
+
 template <typename T>
 int talloc(rtg_context* ctx, DBuf<T>& b, size_t n, cudaStream_t st, const char* what) {
   b.p = nullptr;
@@ -405,6 +452,16 @@ int talloc(rtg_context* ctx, DBuf<T>& b, size_t n, cudaStream_t st, const char* 
   if (n == 0) return RTG_OK;
   if (injected_alloc_failure(ctx))
     return set_error(ctx, RTG_ERR_OUT_OF_MEMORY, std::string("cudaMallocAsync failed for ") + what + " (injected)");
+  if (ctx->scratch_open && st == ctx->stream) {
+    const size_t at = (ctx->scratch_top + 255) / 256 * 256;
+    if (at <= ctx->scratch.n && n * sizeof(T) <= ctx->scratch.n - at) {
+      b.p = reinterpret_cast<T*>(ctx->scratch.p + at);
+      b.n = n;
+      b.scratch = true;
+      ctx->scratch_top = at + n * sizeof(T);
+      return RTG_OK;
+    }
+  }
   cudaError_t e = cudaMallocAsync((void**)&b.p, n * sizeof(T), st);
   if (e != cudaSuccess) {
     b.p = nullptr;
@@ -416,9 +473,10 @@ int talloc(rtg_context* ctx, DBuf<T>& b, size_t n, cudaStream_t st, const char* 
 }
 template <typename T>
 void tfree(DBuf<T>& b, cudaStream_t st) {
-  if (b.p) cudaFreeAsync(b.p, st);
+  if (b.p && !b.scratch) cudaFreeAsync(b.p, st);  // scratch is taken back as a whole
   b.p = nullptr;
   b.n = 0;
+  b.scratch = false;
 }
 
 // device helpers shared by the kernels

@@ -36,45 +36,64 @@ __device__ __forceinline__ float fdec(uint32_t u) {
 
 // Conservative boxes: the exact extent of the disc (r*sqrt(1-n_i^2)) or of the
 // triangle, padded so that every hit the primitive test accepts lies inside.
-__global__ void prim_bounds_kernel(const float4* __restrict__ dcr, const float4* __restrict__ dn, int64_t nd,
+constexpr int kBoundsThreads = 256;
+__global__ void __launch_bounds__(kBoundsThreads) prim_bounds_kernel(const float4* __restrict__ dcr, const float4* __restrict__ dn, int64_t nd,
                                    const float4* __restrict__ tv, const uint32_t* __restrict__ tidx,
                                    int64_t nt, float* __restrict__ plo, float* __restrict__ phi,
                                    uint32_t* __restrict__ cbounds) {
   int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= nd + nt) return;
-  float lo[3], hi[3];
-  if (p < nd) {
-    float4 c = dcr[p], n = dn[p];
-    float cc[3] = {c.x, c.y, c.z}, nn[3] = {n.x, n.y, n.z};
+  uint32_t cmin[3] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}, cmax[3] = {0u, 0u, 0u};
+  if (p < nd + nt) {
+    float lo[3], hi[3];
+    if (p < nd) {
+      float4 c = dcr[p], n = dn[p];
+      float cc[3] = {c.x, c.y, c.z}, nn[3] = {n.x, n.y, n.z};
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      float e = 1.0f - nn[a] * nn[a];
-      float ext = c.w * sqrtf(e > 0.0f ? e : 0.0f);
-      float pad = 1e-5f * (fabsf(cc[a]) + c.w) + 1e-4f * c.w;
-      lo[a] = cc[a] - ext - pad;
-      hi[a] = cc[a] + ext + pad;
+      for (int a = 0; a < 3; ++a) {
+        float e = 1.0f - nn[a] * nn[a];
+        float ext = c.w * sqrtf(e > 0.0f ? e : 0.0f);
+        float pad = 1e-5f * (fabsf(cc[a]) + c.w) + 1e-4f * c.w;
+        lo[a] = cc[a] - ext - pad;
+        hi[a] = cc[a] + ext + pad;
+      }
+    } else {
+      int64_t t = p - nd;
+      float4 v0 = tv[tidx[3 * t]], v1 = tv[tidx[3 * t + 1]], v2 = tv[tidx[3 * t + 2]];
+      float a0[3] = {v0.x, v0.y, v0.z}, a1[3] = {v1.x, v1.y, v1.z}, a2[3] = {v2.x, v2.y, v2.z};
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        float l = fminf(a0[a], fminf(a1[a], a2[a])), h = fmaxf(a0[a], fmaxf(a1[a], a2[a]));
+        float pad = 1e-5f * (fabsf(l) + fabsf(h)) + 1e-6f * (h - l) + 1e-7f;
+        lo[a] = l - pad;
+        hi[a] = h + pad;
+      }
     }
-  } else {
-    int64_t t = p - nd;
-    float4 v0 = tv[tidx[3 * t]], v1 = tv[tidx[3 * t + 1]], v2 = tv[tidx[3 * t + 2]];
-    float a0[3] = {v0.x, v0.y, v0.z}, a1[3] = {v1.x, v1.y, v1.z}, a2[3] = {v2.x, v2.y, v2.z};
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      float l = fminf(a0[a], fminf(a1[a], a2[a])), h = fmaxf(a0[a], fmaxf(a1[a], a2[a]));
-      float pad = 1e-5f * (fabsf(l) + fabsf(h)) + 1e-6f * (h - l) + 1e-7f;
-      lo[a] = l - pad;
-      hi[a] = h + pad;
+      plo[3 * p + a] = lo[a];
+      phi[3 * p + a] = hi[a];
+      cmin[a] = cmax[a] = fenc(0.5f * (lo[a] + hi[a]));
     }
   }
+  if (!cbounds) return;
+  // one atomic per block and bound (one per primitive kept the L2 atomics busy: 4.2 M discs 0.9 ms)
+  __shared__ uint32_t red[kBoundsThreads / 32][6];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    plo[3 * p + a] = lo[a];
-    phi[3 * p + a] = hi[a];
-    float c = 0.5f * (lo[a] + hi[a]);
-    if (cbounds) {
-      atomicMin(&cbounds[a], fenc(c));
-      atomicMax(&cbounds[3 + a], fenc(c));
+    const uint32_t l = __reduce_min_sync(0xFFFFFFFFu, cmin[a]), h = __reduce_max_sync(0xFFFFFFFFu, cmax[a]);
+    if (lane == 0) {
+      red[warp][a] = l;
+      red[warp][3 + a] = h;
     }
+  }
+  __syncthreads();
+  if (threadIdx.x < 6) {
+    uint32_t v = red[0][threadIdx.x];
+    for (int w = 1; w < kBoundsThreads / 32; ++w)
+      v = threadIdx.x < 3 ? min(v, red[w][threadIdx.x]) : max(v, red[w][threadIdx.x]);
+    if (threadIdx.x < 3) atomicMin(&cbounds[threadIdx.x], v);
+    else atomicMax(&cbounds[threadIdx.x], v);
   }
 }
 
@@ -122,8 +141,9 @@ __global__ void slots_kernel(const uint32_t* __restrict__ sorted_prim, const uin
                              uint32_t* __restrict__ leaf_ref, int32_t* __restrict__ leaf_prim) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= np) return;
-  uint32_t p = sorted_prim[i];
-  uint32_t ds = disc_rank[i];
+  const uint32_t p = min(sorted_prim[i], (uint32_t)(np - 1));  // a failed sort (reported) leaves anything here
+  // discs before this position: all or none of them where there is one kind only
+  const uint32_t ds = disc_rank ? disc_rank[i] : (nd > 0 ? (uint32_t)i : 0u);
   leaf_prim[i] = (int32_t)p;
   if (p < (uint32_t)nd) {
     float4 n = dn_id[p];
@@ -213,7 +233,7 @@ __global__ void ploc_init_kernel(const uint32_t* __restrict__ sorted_prim, int64
                                  float4* __restrict__ bhi) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const int64_t p = sorted_prim[i];
+  const int64_t p = min(sorted_prim[i], (uint32_t)(n - 1));
   cid[i] = kClusterLeaf | (uint32_t)i;
   blo[i] = make_float4(plo[3 * p], plo[3 * p + 1], plo[3 * p + 2], 0.0f);
   bhi[i] = make_float4(phi[3 * p], phi[3 * p + 1], phi[3 * p + 2], 0.0f);
@@ -484,25 +504,80 @@ __global__ void __launch_bounds__(kPlocTailThreads) ploc_tail_kernel(
   }
 }
 
-__device__ __forceinline__ void child_box(uint32_t ref, const float4* __restrict__ dn,
-                                          const float4* __restrict__ tri, const float* __restrict__ plo,
-                                          const float* __restrict__ phi, const float* node_box, float* lo,
-                                          float* hi) {
+// A box on its way up the tree, with the height (binary levels) of its subtree.
+struct __align__(16) NodeBox {
+  float lo[3];
+  int32_t height;
+  float hi[3];
+  int32_t unused;
+};
+
+__device__ __forceinline__ NodeBox child_box(uint32_t ref, const float4* __restrict__ dn,
+                                             const float4* __restrict__ tri, const float* __restrict__ plo,
+                                             const float* __restrict__ phi, const NodeBox* node_box) {
+  NodeBox b;
   if (ref & kLeafBit) {
     uint32_t slot = ref & kSlotMask;
     int p = (ref & kTriBit) ? __float_as_int(tri[4 * (int64_t)slot].w) : __float_as_int(dn[2 * (int64_t)slot + 1].w);
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      lo[a] = plo[3 * (int64_t)p + a];
-      hi[a] = phi[3 * (int64_t)p + a];
+      b.lo[a] = plo[3 * (int64_t)p + a];
+      b.hi[a] = phi[3 * (int64_t)p + a];
     }
-  } else {
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      lo[a] = __ldcg(&node_box[6 * (int64_t)ref + a]);
-      hi[a] = __ldcg(&node_box[6 * (int64_t)ref + 3 + a]);
-    }
+    b.height = 0;
+  } else {  // written by another block: past L1
+    const float4* q = reinterpret_cast<const float4*>(node_box + ref);
+    const float4 l = __ldcg(q), h = __ldcg(q + 1);
+    b.lo[0] = l.x; b.lo[1] = l.y; b.lo[2] = l.z;
+    b.hi[0] = h.x; b.hi[1] = h.y; b.hi[2] = h.z;
+    b.height = __float_as_int(l.w);
   }
+  b.unused = 0;
+  return b;
+}
+
+__device__ __forceinline__ void store_boxes(Node& n, const NodeBox& b0, const NodeBox& b1) {
+  n.a = make_float4(b0.lo[0], b0.hi[0], b1.lo[0], b1.hi[0]);
+  n.b = make_float4(b0.lo[1], b0.hi[1], b1.lo[1], b1.hi[1]);
+  n.c = make_float4(b0.lo[2], b0.hi[2], b1.lo[2], b1.hi[2]);
+}
+
+// What a build reports: errors of the sort, the structure check and the refit,
+// the tree's height, the stack need of its quads.
+enum : int { kStSort = 0, kStCheck, kStRefit, kStHeight, kStNeed, kStWords };
+
+// Bottom-up refit: the second thread to reach a node writes both child boxes.
+// A serial chain of the tree's height, a node costs one atomic that orders the
+// boxes behind it and two dependent loads (a fence on either side of the
+// atomic, scalar box loads and the quad nodes on the same chain took 0.16 ms
+// for 200 k triangles).
+__global__ void refit_kernel(int64_t n, const uint32_t* __restrict__ parent, const float4* __restrict__ dn,
+                             const float4* __restrict__ tri, const float* __restrict__ plo,
+                             const float* __restrict__ phi, Node* nodes, NodeBox* node_box, unsigned int* flags,
+                             unsigned long long* status) {
+  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  uint32_t node = parent[(n - 1) + i];
+  for (int iter = 0; iter < 256; ++iter) {
+    if ((int64_t)node >= n - 1) break;  // a parent that was never written
+    unsigned int old;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(old) : "l"(flags + node) : "memory");
+    if (old == 0) return;
+    const uint4 r = __ldcg(&nodes[node].d);
+    const NodeBox b0 = child_box(r.x, dn, tri, plo, phi, node_box), b1 = child_box(r.y, dn, tri, plo, phi, node_box);
+    store_boxes(nodes[node], b0, b1);
+    const int32_t height = max(b0.height, b1.height) + 1;
+    if (node == 0) {
+      status[kStHeight] = (unsigned long long)height;
+      return;
+    }
+    float4* out = reinterpret_cast<float4*>(node_box + node);
+    out[0] = make_float4(fminf(b0.lo[0], b1.lo[0]), fminf(b0.lo[1], b1.lo[1]), fminf(b0.lo[2], b1.lo[2]),
+                         __int_as_float(height));
+    out[1] = make_float4(fmaxf(b0.hi[0], b1.hi[0]), fmaxf(b0.hi[1], b1.hi[1]), fmaxf(b0.hi[2], b1.hi[2]), 0.0f);
+    node = parent[node];
+  }
+  atomicAdd(&status[kStRefit], 1ull);
 }
 
 // A box as a QuadNode stores it.
@@ -520,255 +595,165 @@ __device__ __forceinline__ QuadBox quad_box(const float* lo, const float* hi) {
   return q;
 }
 
-// What a traversal from a node can need: the low half is the stack entries
-// (inner children but one wait while one is descended into), the high half the
-// node's height in binary levels.
-constexpr int kNeedShift = 16;
-
-// The QuadNode of a binary node from its two children, whose own nodes are
-// complete: as long as there is room, the child of largest surface area is
-// opened, which saves the query a visit.  Opening stops where the stack could
-// outgrow the binary tree's by more than 64 entries (kMaxDepth leaves room for
-// them).  Returns the node's need.
-__device__ int32_t make_quad(QuadNode* out, const Node* nodes, const int32_t* need, uint4 d, const float* l0,
-                             const float* h0, const float* l1, const float* h1) {
-  int32_t height = 0;
-  if (!(d.x & kLeafBit)) height = __ldcg(&need[d.x]) >> kNeedShift;
-  if (!(d.y & kLeafBit)) height = max(height, __ldcg(&need[d.y]) >> kNeedShift);
-  height += 1;
+// The QuadNode of every binary node: its two children and, as long as there is
+// room for `most` boxes, those of the one of largest surface area in its
+// place, which saves the query a visit.
+__global__ void quad_kernel(const Node* __restrict__ nodes, int64_t n_internal, int most, QuadNode* __restrict__ quads) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n_internal) return;
   float lo[4][3], hi[4][3];
   uint32_t ref[4];
-  int n = 0;
-  int32_t stack = 0;
-  for (int most = 4; most >= 2; most -= 2) {
+  auto open = [&](uint32_t node, int k0, int k1) {
+    const Node o = nodes[node];
+    const float box0[6] = {o.a.x, o.b.x, o.c.x, o.a.y, o.b.y, o.c.y};
+    const float box1[6] = {o.a.z, o.b.z, o.c.z, o.a.w, o.b.w, o.c.w};
+#pragma unroll
     for (int a = 0; a < 3; ++a) {
-      lo[0][a] = l0[a];
-      hi[0][a] = h0[a];
-      lo[1][a] = l1[a];
-      hi[1][a] = h1[a];
+      lo[k0][a] = box0[a];
+      hi[k0][a] = box0[3 + a];
+      lo[k1][a] = box1[a];
+      hi[k1][a] = box1[3 + a];
     }
-    ref[0] = d.x;
-    ref[1] = d.y;
-    n = d.x == d.y ? 1 : 2;  // a one-primitive tree holds its leaf in both children of the root
-    while (n > 1 && n < most) {
-      int best = -1;
-      float ba = -1.0f;
-      for (int k = 0; k < n; ++k) {
-        if (ref[k] & kLeafBit) continue;
-        const float x = hi[k][0] - lo[k][0], y = hi[k][1] - lo[k][1], z = hi[k][2] - lo[k][2];
-        const float area = x * y + y * z + z * x;
-        if (area > ba) {
-          ba = area;
-          best = k;
-        }
+    ref[k0] = o.d.x;
+    ref[k1] = o.d.y;
+  };
+  open((uint32_t)i, 0, 1);
+  int n = ref[0] == ref[1] ? 1 : 2;  // a one-primitive tree holds its leaf in both children of the root
+  while (n > 1 && n < most) {
+    int best = -1;
+    float ba = -1.0f;
+    for (int k = 0; k < n; ++k) {
+      if (ref[k] & kLeafBit) continue;
+      const float x = hi[k][0] - lo[k][0], y = hi[k][1] - lo[k][1], z = hi[k][2] - lo[k][2];
+      const float area = x * y + y * z + z * x;
+      if (area > ba) {
+        ba = area;
+        best = k;
       }
-      if (best < 0) break;
-      const Node* o = nodes + ref[best];
-      const float4 a = __ldcg(&o->a), b = __ldcg(&o->b), c = __ldcg(&o->c);
-      const uint4 r = __ldcg(&o->d);
-      const float box0[6] = {a.x, b.x, c.x, a.y, b.y, c.y}, box1[6] = {a.z, b.z, c.z, a.w, b.w, c.w};
-      for (int k = 0; k < 3; ++k) {
-        lo[best][k] = box0[k];
-        hi[best][k] = box0[3 + k];
-        lo[n][k] = box1[k];
-        hi[n][k] = box1[3 + k];
-      }
-      ref[best] = r.x;
-      ref[n] = r.y;
-      ++n;
     }
-    int inner = 0, deepest = 0;
-    for (int k = 0; k < n; ++k)
-      if (!(ref[k] & kLeafBit)) {
-        inner += 1;
-        deepest = max(deepest, __ldcg(&need[ref[k]]) & ((1 << kNeedShift) - 1));
-      }
-    stack = inner > 0 ? deepest + inner - 1 : 0;
-    if (stack <= height + 64) break;
+    if (best < 0 || (int64_t)ref[best] >= n_internal) break;
+    open(ref[best], best, n);
+    ++n;
   }
   QuadBox q[4];
+  uint32_t inner = 0;
   for (int k = 0; k < 4; ++k) {
     if (k < n) {
       q[k] = quad_box(lo[k], hi[k]);
+      if (!(ref[k] & kLeafBit)) inner += 1;
     } else {
-      ref[k] = d.x;
+      ref[k] = kLeafBit;
       for (int a = 0; a < 3; ++a) {
         q[k].c[a] = 0.0f;
         q[k].h[a] = -1e30f;
       }
     }
-    out->xy[k] = make_float4(q[k].c[0], q[k].c[1], q[k].h[0], q[k].h[1]);
   }
-  out->z[0] = make_float4(q[0].c[2], q[1].c[2], q[0].h[2], q[1].h[2]);
-  out->z[1] = make_float4(q[2].c[2], q[3].c[2], q[2].h[2], q[3].h[2]);
-  out->ref = make_uint4(ref[0], ref[1], ref[2], ref[3]);
-  return stack | (height << kNeedShift);
+  QuadNode out;
+  for (int k = 0; k < 4; ++k) out.xy[k] = make_float4(q[k].c[0], q[k].c[1], q[k].h[0], q[k].h[1]);
+  out.z[0] = make_float4(q[0].c[2], q[1].c[2], q[0].h[2], q[1].h[2]);
+  out.z[1] = make_float4(q[2].c[2], q[3].c[2], q[2].h[2], q[3].h[2]);
+  out.ref = make_uint4(ref[0], ref[1], ref[2], ref[3]);
+  out.info = make_uint4(inner, 0u, 0u, 0u);
+  quads[i] = out;
 }
 
-// Bottom-up refit: the second thread to reach a node writes both child boxes
-// and the node's QuadNode.
-__global__ void refit_kernel(int64_t n, const uint32_t* __restrict__ leaf_ref, const uint32_t* __restrict__ parent,
-                             const float4* __restrict__ dn, const float4* __restrict__ tri,
-                             const float* __restrict__ plo, const float* __restrict__ phi, Node* nodes,
-                             QuadNode* quads, float* node_box, int32_t* need, unsigned int* flags,
-                             unsigned long long* status) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  uint32_t node = parent[(n - 1) + i];
-  for (int iter = 0; iter < 256; ++iter) {
-    if ((int64_t)node >= n - 1) break;  // a parent that was never written
-    __threadfence();
-    unsigned int old = atomicAdd(&flags[node], 1u);
-    if (old == 0) return;
-    uint4 r = __ldcg(&nodes[node].d);
-    float l0[3], h0[3], l1[3], h1[3];
-    child_box(r.x, dn, tri, plo, phi, node_box, l0, h0);
-    child_box(r.y, dn, tri, plo, phi, node_box, l1, h1);
-    nodes[node].a = make_float4(l0[0], h0[0], l1[0], h1[0]);
-    nodes[node].b = make_float4(l0[1], h0[1], l1[1], h1[1]);
-    nodes[node].c = make_float4(l0[2], h0[2], l1[2], h1[2]);
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      node_box[6 * (int64_t)node + a] = fminf(l0[a], l1[a]);
-      node_box[6 * (int64_t)node + 3 + a] = fmaxf(h0[a], h1[a]);
+// The deepest stack that a traversal of the quads can need: on the way down to
+// a leaf, the inner children but one wait at every quad.  One thread per leaf:
+// up to the root for the path, then down along the quads on it.
+__global__ void quad_need_kernel(int64_t n, const uint32_t* __restrict__ parent, const QuadNode* __restrict__ quads,
+                                 unsigned long long* __restrict__ status) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  unsigned int need = 0;
+  if (i < n) {
+    uint32_t path[kMaxDepth];
+    int len = 0;
+    uint32_t node = parent[(n - 1) + i];
+    bool whole = false;
+    while (len < kMaxDepth && (int64_t)node < n - 1) {
+      path[len++] = node;
+      if (node == 0) {
+        whole = true;
+        break;
+      }
+      node = parent[node];
     }
-    need[node] = make_quad(quads + node, nodes, need, r, l0, h0, l1, h1);
-    __threadfence();
-    if (node == 0) {
-      status[1] = (unsigned long long)(need[0] & ((1 << kNeedShift) - 1));
-      return;
+    int at = whole ? len - 1 : -1;  // path[at] is the quad to leave; a broken link is the refit's error
+    while (at > 0) {
+      const uint4 r = quads[path[at]].ref;
+      const unsigned int inner = quads[path[at]].info.x;
+      int next = -1;
+      for (int k = at - 1; k >= 0 && k >= at - 3; --k)
+        if (r.x == path[k] || r.y == path[k] || r.z == path[k] || r.w == path[k]) {
+          next = k;
+          break;
+        }
+      if (next < 0) break;  // the leaf itself is a child of this quad
+      need += inner - 1;
+      at = next;
     }
-    node = parent[node];
   }
-  atomicAdd(&status[0], 1ull);
+  need = __reduce_max_sync(0xFFFFFFFFu, need);
+  if ((threadIdx.x & 31) == 0 && need) atomicMax(&status[kStNeed], (unsigned long long)need);
 }
 
 // Structural check of the tree before any traversal: every child reference is
 // in range, and every node except the root has exactly one parent.
+// parents: [internal nodes | discs | triangles].
 __global__ void validate_kernel(const Node* __restrict__ nodes, int64_t n_internal, int64_t nd, int64_t nt,
-                                unsigned int* __restrict__ parents_internal,
-                                unsigned int* __restrict__ parents_disc, unsigned int* __restrict__ parents_tri,
-                                unsigned long long* __restrict__ errors) {
+                                unsigned int* __restrict__ parents, unsigned long long* __restrict__ errors) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_internal) return;
   const uint4 d = nodes[i].d;
   const uint32_t ch[2] = {d.x, d.y};
   for (int k = 0; k < 2; ++k) {
     const uint32_t r = ch[k];
-    const uint32_t slot = r & kSlotMask;
+    const int64_t slot = r & kSlotMask;
+    int64_t at = -1;
     if (r & kLeafBit) {
-      if (r & kTriBit) {
-        if ((int64_t)slot < nt) atomicAdd(&parents_tri[slot], 1u);
-        else atomicAdd(errors, 1ull);
-      } else {
-        if ((int64_t)slot < nd) atomicAdd(&parents_disc[slot], 1u);
-        else atomicAdd(errors, 1ull);
-      }
-    } else if (r & kTriBit) {
-      atomicAdd(errors, 1ull);
-    } else if (slot == 0 || (int64_t)slot >= n_internal) {
-      atomicAdd(errors, 1ull);
-    } else {
-      atomicAdd(&parents_internal[slot], 1u);
+      if (r & kTriBit) at = slot < nt ? n_internal + nd + slot : -1;
+      else at = slot < nd ? n_internal + slot : -1;
+    } else if (!(r & kTriBit) && slot != 0 && slot < n_internal) {
+      at = slot;
     }
+    if (at >= 0) atomicAdd(&parents[at], 1u);
+    else atomicAdd(errors, 1ull);
   }
 }
 
-__global__ void count_check_kernel(const unsigned int* __restrict__ c, int64_t n, unsigned int expect_first,
+// Every entry has one parent but the root (entry 0), which has none.
+__global__ void count_check_kernel(const unsigned int* __restrict__ c, int64_t n,
                                    unsigned long long* __restrict__ errors) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const unsigned int want = i == 0 ? expect_first : 1u;
-  if (c[i] != want) atomicAdd(errors, 1ull);
+  if (c[i] != (i == 0 ? 0u : 1u)) atomicAdd(errors, 1ull);
 }
 
 __global__ void single_leaf_kernel(const uint32_t* __restrict__ leaf_ref, const float4* __restrict__ dn,
                                    const float4* __restrict__ tri, const float* __restrict__ plo,
-                                   const float* __restrict__ phi, Node* nodes, QuadNode* quads) {
+                                   const float* __restrict__ phi, Node* nodes) {
   uint32_t r = leaf_ref[0];
-  float l[3], h[3];
-  child_box(r, dn, tri, plo, phi, nullptr, l, h);
-  make_quad(quads, nodes, nullptr, make_uint4(r, r, 0u, 0u), l, h, l, h);
-  nodes[0].a = make_float4(l[0], h[0], l[0], h[0]);
-  nodes[0].b = make_float4(l[1], h[1], l[1], h[1]);
-  nodes[0].c = make_float4(l[2], h[2], l[2], h[2]);
+  const NodeBox b = child_box(r, dn, tri, plo, phi, nullptr);
+  store_boxes(nodes[0], b, b);
   nodes[0].d = make_uint4(r, r, 0u, 0u);
-}
-
-// Internal nodes from each leaf up to the root (bounded walk); the maximum
-// is the deepest stack a traversal can need.
-__global__ void depth_kernel(int64_t n, const uint32_t* __restrict__ parent, unsigned int* __restrict__ depth) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  uint32_t node = parent[(n - 1) + i];
-  unsigned int d = 0;
-  for (int iter = 0; iter < 512; ++iter) {
-    if ((int64_t)node >= n - 1) {
-      d = 0xFFFFFFFFu;  // a broken link (the structural check reports it)
-      break;
-    }
-    d += 1;
-    if (node == 0) break;
-    node = parent[node];
-  }
-  atomicMax(depth, d);
 }
 
 inline unsigned blocks_for(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
-int tree_depth(rtg_context* ctx, cudaStream_t st) {
+// Enqueues the structure check of the links.
+int check_tree(rtg_context* ctx, unsigned long long* status, cudaStream_t st) {
   Geometry& g = ctx->g;
-  const int64_t np = g.nd + g.nt;
-  if (np < 2) {
-    g.depth = 1;
-    return RTG_OK;
-  }
-  DBuf<unsigned int> dd;
-  RTG_TRY(talloc(ctx, dd, 1, st, "tree depth"));
-  unsigned int h = 0;
-  cudaMemsetAsync(dd.p, 0, sizeof(unsigned int), st);
-  depth_kernel<<<blocks_for(np, 256), 256, 0, st>>>(np, g.parent.p, dd.p);
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&h, dd.p, sizeof h, cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  tfree(dd, st);
-  if (e != cudaSuccess) return check_cuda(ctx, e, "tree depth");
-  if (h > (unsigned)kMaxDepth) return set_error(ctx, RTG_ERR_INTERNAL, "LBVH deeper than 192 levels");
-  g.depth = (int32_t)h;
-  return RTG_OK;
-}
-
-int validate_tree(rtg_context* ctx, cudaStream_t st) {
-  Geometry& g = ctx->g;
-  const int64_t np = g.nd + g.nt;
+  const int64_t np = g.nd + g.nt, ni = np - 1;
   if (np < 2) return RTG_OK;
-  const int64_t ni = np - 1;
-  DBuf<unsigned int> pi, pd, pt;
-  DBuf<unsigned long long> err;
-  auto cleanup = [&]() { tfree(pi, st); tfree(pd, st); tfree(pt, st); tfree(err, st); };
-  int rc = talloc(ctx, pi, (size_t)ni, st, "tree check");
-  if (rc == RTG_OK) rc = talloc(ctx, pd, (size_t)(g.nd ? g.nd : 1), st, "tree check");
-  if (rc == RTG_OK) rc = talloc(ctx, pt, (size_t)(g.nt ? g.nt : 1), st, "tree check");
-  if (rc == RTG_OK) rc = talloc(ctx, err, 1, st, "tree check");
-  if (rc != RTG_OK) { cleanup(); return rc; }
-  cudaMemsetAsync(pi.p, 0, ni * sizeof(unsigned int), st);
-  cudaMemsetAsync(pd.p, 0, pd.n * sizeof(unsigned int), st);
-  cudaMemsetAsync(pt.p, 0, pt.n * sizeof(unsigned int), st);
-  cudaMemsetAsync(err.p, 0, sizeof(unsigned long long), st);
-  validate_kernel<<<blocks_for(ni, 256), 256, 0, st>>>(g.nodes.p, ni, g.nd, g.nt, pi.p, pd.p, pt.p, err.p);
-  count_check_kernel<<<blocks_for(ni, 256), 256, 0, st>>>(pi.p, ni, 0u, err.p);
-  if (g.nd) count_check_kernel<<<blocks_for(g.nd, 256), 256, 0, st>>>(pd.p, g.nd, 1u, err.p);
-  if (g.nt) count_check_kernel<<<blocks_for(g.nt, 256), 256, 0, st>>>(pt.p, g.nt, 1u, err.p);
-  unsigned long long h = 0;
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&h, err.p, sizeof h, cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  cleanup();
-  if (e != cudaSuccess) return check_cuda(ctx, e, "LBVH check");
-  if (h) return set_error(ctx, RTG_ERR_INTERNAL, "LBVH check failed: " + std::to_string(h) + " bad links");
+  DBuf<unsigned int> parents;
+  RTG_TRY(talloc(ctx, parents, (size_t)(ni + np), st, "tree check"));
+  cudaMemsetAsync(parents.p, 0, (size_t)(ni + np) * sizeof(unsigned int), st);
+  validate_kernel<<<blocks_for(ni, 256), 256, 0, st>>>(g.nodes.p, ni, g.nd, g.nt, parents.p, status + kStCheck);
+  count_check_kernel<<<blocks_for(ni + np, 256), 256, 0, st>>>(parents.p, ni + np, status + kStCheck);
+  tfree(parents, st);
+  RTG_CUDA(ctx, cudaGetLastError());
   return RTG_OK;
 }
-
 
 // Binary tree over the np sorted leaves by PLOC (see ploc_* kernels): writes
 // the child references of nodes [0, np-1) and the parent array; boxes come
@@ -861,61 +846,95 @@ int run_bounds(rtg_context* ctx, uint32_t* d_cbounds, cudaStream_t st) {
   const int64_t np = g.nd + g.nt;
   RTG_TRY(dalloc(ctx, g.prim_lo, (size_t)(3 * np), "primitive boxes"));
   RTG_TRY(dalloc(ctx, g.prim_hi, (size_t)(3 * np), "primitive boxes"));
-  prim_bounds_kernel<<<blocks_for(np, 256), 256, 0, st>>>(g.disc_cr_by_id.p, g.disc_n_by_id.p, g.nd,
-                                                          g.tri_v.p, g.tri_idx.p, g.nt, g.prim_lo.p,
-                                                          g.prim_hi.p, d_cbounds);
+  prim_bounds_kernel<<<blocks_for(np, kBoundsThreads), kBoundsThreads, 0, st>>>(
+      g.disc_cr_by_id.p, g.disc_n_by_id.p, g.nd, g.tri_v.p, g.tri_idx.p, g.nt, g.prim_lo.p, g.prim_hi.p, d_cbounds);
   RTG_CUDA(ctx, cudaGetLastError());
   return RTG_OK;
 }
 
-int run_slots_and_refit(rtg_context* ctx, const uint32_t* d_sorted_prim, const uint32_t* d_disc_rank,
-                        cudaStream_t st) {
+// Slot-ordered primitive data from the sorted primitive order.
+int run_slots(rtg_context* ctx, const uint32_t* d_sorted_prim, cudaStream_t st) {
   Geometry& g = ctx->g;
   const int64_t np = g.nd + g.nt;
-  if (d_sorted_prim) {
-    slots_kernel<<<blocks_for(np, 256), 256, 0, st>>>(d_sorted_prim, d_disc_rank, np, g.nd, g.disc_cr_by_id.p,
-                                                      g.disc_n_by_id.p, g.tri_v.p, g.tri_idx.p, g.disc.p,
-                                                      g.disc_slot.p, g.tri.p, g.leaf_ref.p,
-                                                      g.leaf_prim.p);
-    RTG_CUDA(ctx, cudaGetLastError());
+  DBuf<uint32_t> rank;  // discs before each sorted position, where discs and triangles mix
+  if (g.nd > 0 && g.nt > 0) {
+    RTG_TRY(talloc(ctx, rank, (size_t)np, st, "disc ranks"));
+    disc_flag_kernel<<<blocks_for(np, 256), 256, 0, st>>>(d_sorted_prim, np, g.nd, rank.p);
+    const int rc = exclusive_scan_u32(ctx, rank.p, np, nullptr, st);
+    if (rc != RTG_OK) {
+      tfree(rank, st);
+      return rc;
+    }
   }
-  if (np == 1) {
-    RTG_TRY(dalloc(ctx, g.quads, 1, "quad nodes"));
-    single_leaf_kernel<<<1, 1, 0, st>>>(g.leaf_ref.p, g.disc.p, g.tri.p, g.prim_lo.p, g.prim_hi.p, g.nodes.p,
-                                        g.quads.p);
-    RTG_CUDA(ctx, cudaGetLastError());
-    g.quad_stack = 0;
-    g.wide_current = false;
-    return wants_wide(ctx) ? build_wide(ctx, st) : RTG_OK;
-  }
-  DBuf<float> node_box;
-  DBuf<int32_t> need;
-  DBuf<unsigned long long> status;  // [0] errors, [1] stack entries the root's quad can need
-  int rc = talloc(ctx, node_box, (size_t)(6 * (np - 1)), st, "node boxes");
-  if (rc == RTG_OK) rc = talloc(ctx, need, (size_t)(np - 1), st, "stack needs");
-  if (rc == RTG_OK) rc = talloc(ctx, status, 2, st, "refit status");
-  if (rc == RTG_OK) rc = dalloc(ctx, g.refit_flags, (size_t)(np - 1), "refit flags");
-  if (rc == RTG_OK) rc = dalloc(ctx, g.quads, (size_t)(np - 1), "quad nodes");
-  auto cleanup = [&]() { tfree(node_box, st); tfree(need, st); tfree(status, st); };
-  if (rc != RTG_OK) {
-    cleanup();
-    return rc;
-  }
-  cudaMemsetAsync(g.refit_flags.p, 0, sizeof(unsigned int) * (np - 1), st);
-  cudaMemsetAsync(status.p, 0, 2 * sizeof(unsigned long long), st);
-  refit_kernel<<<blocks_for(np, 256), 256, 0, st>>>(np, g.leaf_ref.p, g.parent.p, g.disc.p, g.tri.p,
-                                                    g.prim_lo.p, g.prim_hi.p, g.nodes.p, g.quads.p, node_box.p,
-                                                    need.p, g.refit_flags.p, status.p);
-  cudaError_t e = cudaGetLastError();
-  unsigned long long h[2] = {0, 0};
-  if (e == cudaSuccess) e = cudaMemcpyAsync(h, status.p, sizeof h, cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  cleanup();
-  if (e != cudaSuccess) return check_cuda(ctx, e, "LBVH refit");
-  if (h[0]) return set_error(ctx, RTG_ERR_INTERNAL, "LBVH refit exceeded its depth limit");
-  g.quad_stack = (int32_t)h[1];
+  slots_kernel<<<blocks_for(np, 256), 256, 0, st>>>(d_sorted_prim, rank.p, np, g.nd, g.disc_cr_by_id.p,
+                                                    g.disc_n_by_id.p, g.tri_v.p, g.tri_idx.p, g.disc.p, g.disc_slot.p,
+                                                    g.tri.p, g.leaf_ref.p, g.leaf_prim.p);
+  tfree(rank, st);
+  RTG_CUDA(ctx, cudaGetLastError());
+  return RTG_OK;
+}
+
+// Enqueues the boxes, the quads and their stack need over the current links.
+int run_refit(rtg_context* ctx, unsigned long long* status, cudaStream_t st) {
+  Geometry& g = ctx->g;
+  const int64_t np = g.nd + g.nt, ni = np > 1 ? np - 1 : 1;
   g.wide_current = false;  // the wide tree's boxes follow the binary ones: now, or before a trace that wants it
-  return wants_wide(ctx) ? build_wide(ctx, st) : RTG_OK;
+  RTG_TRY(dalloc(ctx, g.quads, (size_t)ni, "quad nodes"));
+  if (np == 1) {
+    single_leaf_kernel<<<1, 1, 0, st>>>(g.leaf_ref.p, g.disc.p, g.tri.p, g.prim_lo.p, g.prim_hi.p, g.nodes.p);
+    quad_kernel<<<1, 1, 0, st>>>(g.nodes.p, 1, 4, g.quads.p);
+    RTG_CUDA(ctx, cudaGetLastError());
+    return RTG_OK;
+  }
+  DBuf<NodeBox> node_box;
+  RTG_TRY(dalloc(ctx, g.refit_flags, (size_t)ni, "refit flags"));
+  RTG_TRY(talloc(ctx, node_box, (size_t)ni, st, "node boxes"));
+  cudaMemsetAsync(g.refit_flags.p, 0, sizeof(unsigned int) * ni, st);
+  refit_kernel<<<blocks_for(np, 256), 256, 0, st>>>(np, g.parent.p, g.disc.p, g.tri.p, g.prim_lo.p, g.prim_hi.p,
+                                                    g.nodes.p, node_box.p, g.refit_flags.p, status);
+  tfree(node_box, st);
+  quad_kernel<<<blocks_for(ni, 128), 128, 0, st>>>(g.nodes.p, ni, 4, g.quads.p);
+  quad_need_kernel<<<blocks_for(np, 256), 256, 0, st>>>(np, g.parent.p, g.quads.p, status);
+  RTG_CUDA(ctx, cudaGetLastError());
+  return RTG_OK;
+}
+
+// Waits for the build and reads its report.
+int read_status(rtg_context* ctx, const unsigned long long* status, unsigned long long* h, cudaStream_t st) {
+  RTG_CUDA(ctx, cudaMemcpyAsync(h, status, kStWords * sizeof *h, cudaMemcpyDeviceToHost, st));
+  RTG_CUDA(ctx, cudaStreamSynchronize(st));
+  return RTG_OK;
+}
+
+// Takes over the height and the stack need of a good build.  Quads that could
+// outgrow the largest stack (a clustering with many inner siblings down a deep
+// path) are made again of two boxes each, which need no more than the height.
+int take_shape(rtg_context* ctx, const unsigned long long* h, cudaStream_t st) {
+  Geometry& g = ctx->g;
+  const int64_t np = g.nd + g.nt;
+  if (np == 1) {
+    g.depth = 1;
+    g.quad_stack = 0;
+    return RTG_OK;
+  }
+  g.depth = (int32_t)h[kStHeight];
+  g.quad_stack = (int32_t)h[kStNeed];
+  if (g.quad_stack > kMaxStack) {
+    quad_kernel<<<blocks_for(np - 1, 128), 128, 0, st>>>(g.nodes.p, np - 1, 2, g.quads.p);
+    RTG_CUDA(ctx, cudaGetLastError());
+    g.quad_stack = g.depth;
+  }
+  return RTG_OK;
+}
+
+int build_status(rtg_context* ctx, const unsigned long long* h) {
+  if (h[kStSort]) return set_error(ctx, RTG_ERR_INTERNAL, "radix sort did not finish");
+  if (h[kStCheck])
+    return set_error(ctx, RTG_ERR_INTERNAL, "LBVH check failed: " + std::to_string(h[kStCheck]) + " bad links");
+  if (h[kStRefit]) return set_error(ctx, RTG_ERR_INTERNAL, "LBVH refit exceeded its depth limit");
+  if (h[kStHeight] > (unsigned long long)kMaxDepth)
+    return set_error(ctx, RTG_ERR_INTERNAL, "LBVH deeper than 256 levels");
+  return RTG_OK;
 }
 
 }  // namespace
@@ -926,28 +945,21 @@ int build_lbvh(rtg_context* ctx) {
   const int64_t np = g.nd + g.nt;
   if (np <= 0) return set_error(ctx, RTG_ERR_NO_GEOMETRY, "no primitives");
   if (np > (int64_t)kSlotMask) return set_error(ctx, RTG_ERR_INVALID_ARGUMENT, "too many primitives");
-  DBuf<uint32_t> cb, keys, vals, tk, tv, rank;
-  auto cleanup = [&]() { tfree(cb, st); tfree(keys, st); tfree(vals, st); tfree(tk, st); tfree(tv, st); tfree(rank, st); };
+  DBuf<uint32_t> cb, pairs;  // centroid bounds; keys | values | scratch for both
+  DBuf<unsigned long long> status;
+  auto cleanup = [&]() { tfree(cb, st); tfree(pairs, st); tfree(status, st); };
   int rc = RTG_OK;
   do {
     if ((rc = talloc(ctx, cb, 6, st, "centroid bounds")) != RTG_OK) break;
-    const uint32_t init[6] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u};
-    if (cudaMemcpyAsync(cb.p, init, sizeof init, cudaMemcpyHostToDevice, st) != cudaSuccess) {
-      rc = check_cuda(ctx, cudaGetLastError(), "centroid bounds init");
-      break;
-    }
+    if ((rc = talloc(ctx, status, kStWords, st, "build status")) != RTG_OK) break;
+    if ((rc = talloc(ctx, pairs, (size_t)(4 * np), st, "morton pairs")) != RTG_OK) break;
+    uint32_t *keys = pairs.p, *vals = pairs.p + np, *tk = pairs.p + 2 * np, *tv = pairs.p + 3 * np;
+    cudaMemsetAsync(cb.p, 0xFF, 3 * sizeof(uint32_t), st);
+    cudaMemsetAsync(cb.p + 3, 0, 3 * sizeof(uint32_t), st);
+    cudaMemsetAsync(status.p, 0, kStWords * sizeof(unsigned long long), st);
     if ((rc = run_bounds(ctx, cb.p, st)) != RTG_OK) break;
-    if ((rc = talloc(ctx, keys, (size_t)np, st, "morton keys")) != RTG_OK) break;
-    if ((rc = talloc(ctx, vals, (size_t)np, st, "morton values")) != RTG_OK) break;
-    if ((rc = talloc(ctx, tk, (size_t)np, st, "sort scratch")) != RTG_OK) break;
-    if ((rc = talloc(ctx, tv, (size_t)np, st, "sort scratch")) != RTG_OK) break;
-    morton_kernel<<<blocks_for(np, 256), 256, 0, st>>>(g.prim_lo.p, g.prim_hi.p, np, cb.p, keys.p, vals.p);
-    if (cudaGetLastError() != cudaSuccess) { rc = check_cuda(ctx, cudaGetLastError(), "morton"); break; }
-    if ((rc = radix_sort_pairs(ctx, keys.p, vals.p, tk.p, tv.p, np, 30, st)) != RTG_OK) break;
-    // disc slot = number of discs before this sorted position
-    if ((rc = talloc(ctx, rank, (size_t)np, st, "disc ranks")) != RTG_OK) break;
-    disc_flag_kernel<<<blocks_for(np, 256), 256, 0, st>>>(vals.p, np, g.nd, rank.p);
-    if ((rc = exclusive_scan_u32(ctx, rank.p, np, nullptr, st)) != RTG_OK) break;
+    morton_kernel<<<blocks_for(np, 256), 256, 0, st>>>(g.prim_lo.p, g.prim_hi.p, np, cb.p, keys, vals);
+    if ((rc = radix_sort_pairs(ctx, keys, vals, tk, tv, np, 30, status.p + kStSort, st)) != RTG_OK) break;
     if ((rc = dalloc(ctx, g.disc, (size_t)(2 * (g.nd ? g.nd : 1)), "disc slots")) != RTG_OK) break;
     if ((rc = dalloc(ctx, g.disc_slot, (size_t)(g.nd ? g.nd : 1), "disc slot map")) != RTG_OK) break;
     if ((rc = dalloc(ctx, g.tri, (size_t)(4 * (g.nt ? g.nt : 1)), "triangle slots")) != RTG_OK) break;
@@ -956,39 +968,33 @@ int build_lbvh(rtg_context* ctx) {
     const int64_t nn = np > 1 ? np - 1 : 1;
     if ((rc = dalloc(ctx, g.nodes, (size_t)nn, "LBVH nodes")) != RTG_OK) break;
     if ((rc = dalloc(ctx, g.parent, (size_t)(2 * np), "LBVH parents")) != RTG_OK) break;
-    // slots first: the Karras kernel reads the leaf references
-    slots_kernel<<<blocks_for(np, 256), 256, 0, st>>>(vals.p, rank.p, np, g.nd, g.disc_cr_by_id.p,
-                                                      g.disc_n_by_id.p, g.tri_v.p, g.tri_idx.p, g.disc.p,
-                                                      g.disc_slot.p, g.tri.p, g.leaf_ref.p,
-                                                      g.leaf_prim.p);
-    if (cudaGetLastError() != cudaSuccess) { rc = check_cuda(ctx, cudaGetLastError(), "slots"); break; }
-    if (np > 1) {
-      // PLOC first; a clustering deeper than the traversal stacks allow (possible
-      // for degenerate inputs) falls back to the Karras tree, whose depth is
-      // bounded by the key length
-      bool karras = g.builder != kBuilderPloc;
-      if (!karras) {
+    // slots first: the builders read the leaf references
+    if ((rc = run_slots(ctx, vals, st)) != RTG_OK) break;
+    unsigned long long h[kStWords] = {};
+    // PLOC first; a clustering deeper than the traversal stacks allow (possible
+    // for degenerate inputs) falls back to the Karras tree, whose depth is
+    // bounded by the key length
+    for (bool karras = g.builder != kBuilderPloc || np == 1;; karras = true) {
+      if (np > 1) {
         cudaMemsetAsync(g.parent.p, 0xFF, 2 * np * sizeof(uint32_t), st);
-        if ((rc = build_ploc(ctx, vals.p, st)) != RTG_OK) break;
-        if ((rc = validate_tree(ctx, st)) != RTG_OK) break;
-        const int drc = tree_depth(ctx, st);  // RTG_ERR_INTERNAL: too deep for the stacks
-        if (drc != RTG_OK && drc != RTG_ERR_INTERNAL) {
-          rc = drc;
+        if (karras) {
+          karras_kernel<<<blocks_for(np - 1, 256), 256, 0, st>>>(keys, np, g.leaf_ref.p, g.nodes.p, g.parent.p);
+        } else if ((rc = build_ploc(ctx, vals, st)) != RTG_OK) {
           break;
         }
-        karras = drc != RTG_OK;
+        if ((rc = check_tree(ctx, status.p, st)) != RTG_OK) break;
       }
-      if (karras) {
-        cudaMemsetAsync(g.parent.p, 0xFF, 2 * np * sizeof(uint32_t), st);
-        karras_kernel<<<blocks_for(np - 1, 256), 256, 0, st>>>(keys.p, np, g.leaf_ref.p, g.nodes.p, g.parent.p);
-        if (cudaGetLastError() != cudaSuccess) { rc = check_cuda(ctx, cudaGetLastError(), "karras"); break; }
-        if ((rc = validate_tree(ctx, st)) != RTG_OK) break;
-      }
+      if ((rc = run_refit(ctx, status.p, st)) != RTG_OK) break;
+      if ((rc = read_status(ctx, status.p, h, st)) != RTG_OK) break;
+      const bool deep = h[kStRefit] != 0 || h[kStHeight] > (unsigned long long)kMaxDepth;
+      if (karras || h[kStSort] || h[kStCheck] || !deep) break;
+      cudaMemsetAsync(status.p, 0, kStWords * sizeof(unsigned long long), st);
     }
-    if ((rc = tree_depth(ctx, st)) != RTG_OK) break;
-    rc = run_slots_and_refit(ctx, nullptr, nullptr, st);
+    if (rc == RTG_OK) rc = build_status(ctx, h);
+    if (rc == RTG_OK) rc = take_shape(ctx, h, st);
+    if (rc == RTG_OK && wants_wide(ctx)) rc = build_wide(ctx, st);
   } while (0);
-  cudaStreamSynchronize(st);
+  if (rc != RTG_OK) cudaStreamSynchronize(st);
   cleanup();
   g.root = 0;
   return rc;
@@ -1000,18 +1006,24 @@ int refit_lbvh(rtg_context* ctx) {
   RTG_TRY(run_bounds(ctx, nullptr, st));
   // keep the leaf order: recompute slot data from the sorted primitive order
   const int64_t np = g.nd + g.nt;
-  DBuf<uint32_t> rank, order;
-  int rc = talloc(ctx, rank, (size_t)np, st, "disc ranks");
-  if (rc == RTG_OK) rc = talloc(ctx, order, (size_t)np, st, "leaf order");
+  DBuf<uint32_t> order;
+  DBuf<unsigned long long> status;
+  int rc = talloc(ctx, order, (size_t)np, st, "leaf order");
+  if (rc == RTG_OK) rc = talloc(ctx, status, kStWords, st, "build status");
+  unsigned long long h[kStWords] = {};
   if (rc == RTG_OK) {
     cudaMemcpyAsync(order.p, g.leaf_prim.p, np * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st);
-    disc_flag_kernel<<<blocks_for(np, 256), 256, 0, st>>>(order.p, np, g.nd, rank.p);
-    rc = exclusive_scan_u32(ctx, rank.p, np, nullptr, st);
+    cudaMemsetAsync(status.p, 0, kStWords * sizeof(unsigned long long), st);
+    rc = run_slots(ctx, order.p, st);
   }
-  if (rc == RTG_OK) rc = run_slots_and_refit(ctx, order.p, rank.p, st);
-  cudaStreamSynchronize(st);
-  tfree(rank, st);
+  if (rc == RTG_OK) rc = run_refit(ctx, status.p, st);
+  if (rc == RTG_OK) rc = read_status(ctx, status.p, h, st);
+  if (rc == RTG_OK) rc = build_status(ctx, h);
+  if (rc == RTG_OK) rc = take_shape(ctx, h, st);
+  if (rc == RTG_OK && wants_wide(ctx)) rc = build_wide(ctx, st);
+  if (rc != RTG_OK) cudaStreamSynchronize(st);
   tfree(order, st);
+  tfree(status, st);
   return rc;
 }
 

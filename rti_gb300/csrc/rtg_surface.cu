@@ -1,7 +1,8 @@
 // rtg_surface.cu -- per-element kernels around the trace:
 //   * neighbour lists of overlapping discs (disc_neighborhood.hpp:20-220):
-//     uniform grid of cell size 2*r_max, each disc tests the 27 surrounding
-//     cells with the reference's predicate distance(c_i, c_j) < r_i + r_j;
+//     uniform grid of cell size 2*r_max, discs counted into its cells and
+//     copied in cell order, each disc tests the 27 surrounding cells (nine runs
+//     of three) with the reference's predicate distance(c_i, c_j) < r_i + r_j;
 //     rows are sorted by id (CSR);
 //   * exposed disc area inside the x/y box (disc_bounding_box_intersector.hpp:
 //     43-441) and triangle areas (utils.hpp:161-169), one thread per element;
@@ -22,34 +23,39 @@ inline unsigned blocks_for(int64_t n, int t) { return (unsigned)((n + t - 1) / t
 
 struct Grid {
   float org[3];
-  float h;
+  float inv_h;
   int dim[3];
 };
 
-__device__ __forceinline__ int cell_coord(float v, float org, float h, int dim) {
-  int c = (int)floor(((double)v - (double)org) / (double)h);
+// Monotone in v, and off by less than 2^-23 * dim cells.
+__device__ __forceinline__ int cell_coord(float v, float org, float inv_h, int dim) {
+  const int c = (int)floorf((v - org) * inv_h);
   return c < 0 ? 0 : (c >= dim ? dim - 1 : c);
 }
 
-__global__ void cell_key_kernel(const float4* __restrict__ dcr, int64_t nd, Grid g, uint32_t* __restrict__ keys,
-                                uint32_t* __restrict__ vals) {
+// The cell of every disc and its place among that cell's discs.
+__global__ void cell_count_kernel(const float4* __restrict__ dcr, int64_t nd, Grid g, uint32_t* __restrict__ count,
+                                  uint2* __restrict__ cell_rank) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nd) return;
-  float4 c = dcr[i];
-  int cx = cell_coord(c.x, g.org[0], g.h, g.dim[0]);
-  int cy = cell_coord(c.y, g.org[1], g.h, g.dim[1]);
-  int cz = cell_coord(c.z, g.org[2], g.h, g.dim[2]);
-  keys[i] = (uint32_t)((cz * g.dim[1] + cy) * g.dim[0] + cx);
-  vals[i] = (uint32_t)i;
+  const float4 c = dcr[i];
+  const int cx = cell_coord(c.x, g.org[0], g.inv_h, g.dim[0]);
+  const int cy = cell_coord(c.y, g.org[1], g.inv_h, g.dim[1]);
+  const int cz = cell_coord(c.z, g.org[2], g.inv_h, g.dim[2]);
+  const uint32_t cell = (uint32_t)((cz * g.dim[1] + cy) * g.dim[0] + cx);
+  cell_rank[i] = make_uint2(cell, atomicAdd(&count[cell], 1u));
 }
 
-__global__ void cell_range_kernel(const uint32_t* __restrict__ keys, int64_t nd, uint32_t* __restrict__ start,
-                                  uint32_t* __restrict__ end) {
+// The discs in cell order (`start`: the exclusive scan of the counts).
+__global__ void cell_place_kernel(const float4* __restrict__ dcr, int64_t nd, const uint32_t* __restrict__ start,
+                                  const uint2* __restrict__ cell_rank, float4* __restrict__ cell_disc,
+                                  uint32_t* __restrict__ cell_id) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nd) return;
-  uint32_t k = keys[i];
-  if (i == 0 || keys[i - 1] != k) start[k] = (uint32_t)i;
-  if (i == nd - 1 || keys[i + 1] != k) end[k] = (uint32_t)(i + 1);
+  const uint2 cr = cell_rank[i];
+  const uint32_t at = start[cr.x] + cr.y;
+  cell_disc[at] = dcr[i];
+  cell_id[at] = (uint32_t)i;
 }
 
 // check_dist (disc_neighborhood.hpp:190-220): the three axis pre-tests are
@@ -60,53 +66,61 @@ __device__ __forceinline__ bool overlaps(float4 a, float4 b) {
   return dist < a.w + b.w;
 }
 
-template <bool kFill>
-__global__ void neighbor_kernel(const float4* __restrict__ dcr, int64_t nd, Grid g,
-                                const uint32_t* __restrict__ sorted_ids, const uint32_t* __restrict__ start,
-                                const uint32_t* __restrict__ end, int64_t* __restrict__ counts,
-                                const int64_t* __restrict__ row_ptr, int32_t* __restrict__ cols) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nd) return;
-  const float4 ci = dcr[i];
-  const int cx = cell_coord(ci.x, g.org[0], g.h, g.dim[0]);
-  const int cy = cell_coord(ci.y, g.org[1], g.h, g.dim[1]);
-  const int cz = cell_coord(ci.z, g.org[2], g.h, g.dim[2]);
+// One thread per disc, in cell order (the lanes of a warp read the same runs).
+// FILL = false: the row's length; FILL = true: the row, sorted by id, as ids and
+// as disc slots.  Bound by the latency of the nine runs' loads; cells of 2 r_max
+// (up to 16 a disc) instead of fewer, wider ones, discs copied in cell order and
+// rows sorted in the thread took the pair of launches from 0.15 to 0.06 ms on
+// 98 k discs and from 22 to 1.3 ms on 4.19 M.
+template <bool FILL>
+__global__ void neighbor_kernel(const float4* __restrict__ cell_disc, const uint32_t* __restrict__ cell_id, int64_t nd,
+                                Grid g, const uint32_t* __restrict__ start, int64_t* __restrict__ row,
+                                const uint32_t* __restrict__ slot_of_id, int32_t* __restrict__ cols,
+                                uint32_t* __restrict__ slots) {
+  const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= nd) return;
+  const float4 ci = cell_disc[s];
+  const uint32_t id = cell_id[s];
+  const int cx = cell_coord(ci.x, g.org[0], g.inv_h, g.dim[0]);
+  const int cy = cell_coord(ci.y, g.org[1], g.inv_h, g.dim[1]);
+  const int cz = cell_coord(ci.z, g.org[2], g.inv_h, g.dim[2]);
+  const int x0 = max(cx - 1, 0), x1 = min(cx + 1, g.dim[0] - 1);
+  constexpr int kLocal = 32;  // longer rows are sorted where they lie
+  int32_t buf[FILL ? kLocal : 1];
+  const int64_t out = FILL ? row[id] : 0;
+  const int64_t len = FILL ? row[id + 1] - out : 0;
+  const bool local = len <= kLocal;
   int64_t cnt = 0;
-  int64_t out = kFill ? row_ptr[i] : 0;
-  for (int z = cz - 1; z <= cz + 1; ++z) {
-    if (z < 0 || z >= g.dim[2]) continue;
-    for (int y = cy - 1; y <= cy + 1; ++y) {
-      if (y < 0 || y >= g.dim[1]) continue;
-      for (int x = cx - 1; x <= cx + 1; ++x) {
-        if (x < 0 || x >= g.dim[0]) continue;
-        const uint32_t cell = (uint32_t)((z * g.dim[1] + y) * g.dim[0] + x);
-        const uint32_t b = start[cell];
-        if (b == 0xFFFFFFFFu) continue;
-        const uint32_t e = end[cell];
-        for (uint32_t q = b; q < e; ++q) {
-          const uint32_t j = sorted_ids[q];
-          if (j == (uint32_t)i) continue;
-          if (overlaps(ci, dcr[j])) {
-            if (kFill) cols[out + cnt] = (int32_t)j;
-            ++cnt;
+  for (int z = max(cz - 1, 0); z <= min(cz + 1, g.dim[2] - 1); ++z)
+    for (int y = max(cy - 1, 0); y <= min(cy + 1, g.dim[1] - 1); ++y) {
+      const int64_t line = ((int64_t)z * g.dim[1] + y) * g.dim[0];
+      const uint32_t b = start[line + x0], e = start[line + x1 + 1];
+      for (uint32_t q = b; q < e; ++q) {
+        if (q == (uint32_t)s || !overlaps(ci, cell_disc[q])) continue;
+        if (FILL) {
+          if (cnt >= len) continue;  // cannot happen: the same test counted the row
+          const int32_t j = (int32_t)cell_id[q];
+          if (local) {  // insertion by id
+            int k = (int)cnt;
+            for (; k > 0 && buf[k - 1] > j; --k) buf[k] = buf[k - 1];
+            buf[k] = j;
+          } else {
+            int64_t k = out + cnt;
+            for (; k > out && cols[k - 1] > j; --k) cols[k] = cols[k - 1];
+            cols[k] = j;
           }
         }
+        ++cnt;
       }
     }
-  }
-  if (kFill) {
-    // insertion sort of the row by id
-    for (int64_t a = out + 1; a < out + cnt; ++a) {
-      int32_t v = cols[a];
-      int64_t b = a - 1;
-      while (b >= out && cols[b] > v) {
-        cols[b + 1] = cols[b];
-        --b;
-      }
-      cols[b + 1] = v;
+  if (FILL) {
+    for (int64_t k = 0; k < len; ++k) {
+      const int32_t j = local ? buf[k] : cols[out + k];
+      if (local) cols[out + k] = j;
+      slots[out + k] = slot_of_id[j];
     }
   } else {
-    counts[i] = cnt;
+    row[id] = cnt;
   }
 }
 
@@ -284,17 +298,30 @@ __global__ void area_kernel(const float4* __restrict__ dcr, const float4* __rest
 }
 
 // ---------------- normalised smoothed estimates (device.hpp:154-187) --------
-__global__ void smooth_kernel(const double* __restrict__ s1, const float* __restrict__ areas, int64_t n,
-                              int64_t nd, const int64_t* __restrict__ rp, const int32_t* __restrict__ cols,
-                              float* __restrict__ est, unsigned long long* __restrict__ maxbits) {
+// S1 per area of every disc: a disc's value is read once for itself and once
+// for every neighbour, and the FP64 division is what these kernels wait for
+// (98 k discs: 37 us with a division per neighbour, now 6 + 8).
+__global__ void flux_kernel(const double* __restrict__ s1, const float* __restrict__ areas, int64_t nd,
+                            double* __restrict__ flux) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < nd) flux[i] = s1[i] / areas[i];
+}
+
+__global__ void smooth_kernel(const double* __restrict__ s1, const float* __restrict__ areas,
+                              const double* __restrict__ flux, int64_t n, int64_t nd, const int64_t* __restrict__ rp,
+                              const int32_t* __restrict__ cols, float* __restrict__ est,
+                              unsigned long long* __restrict__ maxbits) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   double vv = 0.0;
   if (i < n) {
-    vv = s1[i] / areas[i];
     int64_t deg = 0;
-    if (rp && i < nd) {
-      for (int64_t q = rp[i]; q < rp[i + 1]; ++q) vv += s1[cols[q]] / areas[cols[q]];
-      deg = rp[i + 1] - rp[i];
+    if (i < nd) {
+      vv = flux[i];
+      const int64_t q0 = rp[i], q1 = rp[i + 1];
+      for (int64_t q = q0; q < q1; ++q) vv += flux[cols[q]];
+      deg = q1 - q0;
+    } else {
+      vv = s1[i] / areas[i];
     }
     vv /= (double)(deg + 1);
     est[i] = (float)vv;
@@ -344,89 +371,97 @@ __global__ void stats_kernel(const double* __restrict__ s1, const double* __rest
 
 }  // namespace
 
-// Neighbour columns as disc slots, for the trace (one 256-bit record load per neighbour).
-__global__ void nb_slot_kernel(const int32_t* __restrict__ nb_idx, int64_t nnz, const uint32_t* __restrict__ slot_of_id,
-                               uint32_t* __restrict__ nb_slot) {
-  int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q < nnz) nb_slot[q] = slot_of_id[nb_idx[q]];
-}
-
-int build_neighbors(rtg_context* ctx) {
+// Enqueues the discs' cells and the row lengths, scanned into nb_ptr: needs the
+// discs by id only, so that it runs before the tree is there.
+int count_neighbors(rtg_context* ctx, NeighborWork& w) {
   Geometry& g = ctx->g;
   cudaStream_t st = ctx->stream;
   const int64_t nd = g.nd;
   g.nb_nnz = 0;
   RTG_TRY(dalloc(ctx, g.nb_ptr, (size_t)(nd + 1), "neighbour row pointers"));
   if (nd == 0) return RTG_OK;
+  RTG_CUDA(ctx, cudaMemsetAsync(g.nb_ptr.p + nd, 0, sizeof(int64_t), st));
   if (nd == 1) {
-    RTG_CUDA(ctx, cudaMemsetAsync(g.nb_ptr.p, 0, 2 * sizeof(int64_t), st));
-    RTG_TRY(dalloc(ctx, g.nb_idx, 1, "neighbour columns"));
-    RTG_TRY(dalloc(ctx, g.nb_slot, 1, "neighbour slots"));
+    RTG_CUDA(ctx, cudaMemsetAsync(g.nb_ptr.p, 0, sizeof(int64_t), st));
     return RTG_OK;
   }
+  // A cell is 1 % wider than the largest distance of an overlap, far more than
+  // the rounding of a coordinate (below 2^-8 cells for up to 2^14 a side), so
+  // overlapping discs lie at most one cell apart.
   Grid grid;
-  float h = 2.0f * g.rmax * 1.000001f;
-  if (!(h > 0.0f)) h = 1.0f;
+  double h = 2.02 * (double)g.rmax;
+  if (!(h > 0.0)) h = 1.0;
   double ext[3];
   for (int a = 0; a < 3; ++a) ext[a] = (double)g.cmax[a] - (double)g.cmin[a];
-  // cap the number of cells near 2 per disc; larger cells keep the test exact
+  // at most 16 cells a disc; larger cells keep the test exact
   for (;;) {
     double cells = 1.0;
-    for (int a = 0; a < 3; ++a) cells *= std::floor(ext[a] / h) + 1.0;
-    if (cells <= 2.0 * (double)nd + 64.0 && cells < 2.0e9) break;
-    h *= 1.25f;
+    bool fits = true;
+    for (int a = 0; a < 3; ++a) {
+      const double n = std::floor(ext[a] / h) + 2.0;
+      fits = fits && n <= 16384.0;
+      cells *= n;
+    }
+    if (fits && cells <= 16.0 * (double)nd + 4096.0 && cells < 2.0e9) break;
+    h *= 1.25;
   }
   for (int a = 0; a < 3; ++a) {
     grid.org[a] = g.cmin[a];
-    grid.dim[a] = (int)std::floor(ext[a] / h) + 1;
+    grid.dim[a] = (int)std::floor(ext[a] / h) + 2;
   }
-  grid.h = h;
+  grid.inv_h = (float)(1.0 / h);
   const int64_t ncells = (int64_t)grid.dim[0] * grid.dim[1] * grid.dim[2];
-  DBuf<uint32_t> keys, vals, tk, tv, cs, ce;
-  DBuf<int64_t> counts;
-  auto cleanup = [&]() { tfree(keys, st); tfree(vals, st); tfree(tk, st); tfree(tv, st); tfree(cs, st); tfree(ce, st); tfree(counts, st); };
-  int rc = RTG_OK;
-  do {
-    if ((rc = talloc(ctx, keys, (size_t)nd, st, "grid keys")) != RTG_OK) break;
-    if ((rc = talloc(ctx, vals, (size_t)nd, st, "grid ids")) != RTG_OK) break;
-    if ((rc = talloc(ctx, tk, (size_t)nd, st, "sort scratch")) != RTG_OK) break;
-    if ((rc = talloc(ctx, tv, (size_t)nd, st, "sort scratch")) != RTG_OK) break;
-    if ((rc = talloc(ctx, cs, (size_t)ncells, st, "cell starts")) != RTG_OK) break;
-    if ((rc = talloc(ctx, ce, (size_t)ncells, st, "cell ends")) != RTG_OK) break;
-    if ((rc = talloc(ctx, counts, (size_t)(nd + 1), st, "neighbour counts")) != RTG_OK) break;
-    cell_key_kernel<<<blocks_for(nd, 256), 256, 0, st>>>(g.disc_cr_by_id.p, nd, grid, keys.p, vals.p);
-    int bits = 1;
-    while (bits < 32 && ((int64_t)1 << bits) < ncells) ++bits;
-    if ((rc = radix_sort_pairs(ctx, keys.p, vals.p, tk.p, tv.p, nd, bits, st)) != RTG_OK) break;
-    cudaMemsetAsync(cs.p, 0xFF, ncells * sizeof(uint32_t), st);
-    cudaMemsetAsync(ce.p, 0x00, ncells * sizeof(uint32_t), st);
-    cell_range_kernel<<<blocks_for(nd, 256), 256, 0, st>>>(keys.p, nd, cs.p, ce.p);
-    neighbor_kernel<false><<<blocks_for(nd, 128), 128, 0, st>>>(g.disc_cr_by_id.p, nd, grid, vals.p, cs.p, ce.p,
-                                                                counts.p, nullptr, nullptr);
-    cudaMemsetAsync(counts.p + nd, 0, sizeof(int64_t), st);
-    int64_t* total = g.nb_ptr.p + nd;
-    if ((rc = exclusive_scan_i64(ctx, counts.p, nd + 1, nullptr, st)) != RTG_OK) break;
-    int64_t nnz = 0;
-    cudaError_t cerr = cudaMemcpyAsync(g.nb_ptr.p, counts.p, (nd + 1) * sizeof(int64_t), cudaMemcpyDeviceToDevice, st);
-    if (cerr == cudaSuccess) cerr = cudaMemcpyAsync(&nnz, total, sizeof(int64_t), cudaMemcpyDeviceToHost, st);
-    if (cerr == cudaSuccess) cerr = cudaStreamSynchronize(st);
-    if (cerr != cudaSuccess) {
-      rc = check_cuda(ctx, cerr, "neighbour counts");
-      break;
-    }
-    g.nb_nnz = nnz;
-    if ((rc = dalloc(ctx, g.nb_idx, (size_t)(nnz > 0 ? nnz : 1), "neighbour columns")) != RTG_OK) break;
-    neighbor_kernel<true><<<blocks_for(nd, 128), 128, 0, st>>>(g.disc_cr_by_id.p, nd, grid, vals.p, cs.p, ce.p,
-                                                               nullptr, g.nb_ptr.p, g.nb_idx.p);
-    if ((rc = dalloc(ctx, g.nb_slot, (size_t)(nnz > 0 ? nnz : 1), "neighbour slots")) != RTG_OK) break;
-    if (nnz > 0)
-      nb_slot_kernel<<<blocks_for(nnz, 256), 256, 0, st>>>(g.nb_idx.p, nnz, g.disc_slot.p, g.nb_slot.p);
-    cudaError_t e = cudaStreamSynchronize(st);
-    if (e == cudaSuccess) e = cudaGetLastError();
-    if (e != cudaSuccess) rc = check_cuda(ctx, e, "neighbour lists");
-  } while (0);
-  cleanup();
-  return rc;
+  RTG_TRY(talloc(ctx, w.start, (size_t)(ncells + 1), st, "grid cells"));
+  RTG_TRY(talloc(ctx, w.cell_rank, (size_t)nd, st, "grid cells"));
+  RTG_TRY(talloc(ctx, w.cell_disc, (size_t)nd, st, "grid discs"));
+  RTG_TRY(talloc(ctx, w.cell_id, (size_t)nd, st, "grid ids"));
+  cudaMemsetAsync(w.start.p, 0, (size_t)(ncells + 1) * sizeof(uint32_t), st);
+  cell_count_kernel<<<blocks_for(nd, 256), 256, 0, st>>>(g.disc_cr_by_id.p, nd, grid, w.start.p, w.cell_rank.p);
+  RTG_TRY(exclusive_scan_u32(ctx, w.start.p, ncells + 1, nullptr, st));
+  cell_place_kernel<<<blocks_for(nd, 256), 256, 0, st>>>(g.disc_cr_by_id.p, nd, w.start.p, w.cell_rank.p,
+                                                         w.cell_disc.p, w.cell_id.p);
+  neighbor_kernel<false><<<blocks_for(nd, 128), 128, 0, st>>>(w.cell_disc.p, w.cell_id.p, nd, grid, w.start.p,
+                                                              g.nb_ptr.p, nullptr, nullptr, nullptr);
+  RTG_CUDA(ctx, cudaGetLastError());
+  RTG_TRY(exclusive_scan_i64(ctx, g.nb_ptr.p, nd + 1, nullptr, st));
+  for (int a = 0; a < 3; ++a) {
+    w.org[a] = grid.org[a];
+    w.dim[a] = grid.dim[a];
+  }
+  w.inv_h = grid.inv_h;
+  return RTG_OK;
+}
+
+// Enqueues the rows, once the tree's slots are there (waits for the row lengths).
+int fill_neighbors(rtg_context* ctx, NeighborWork& w) {
+  Geometry& g = ctx->g;
+  cudaStream_t st = ctx->stream;
+  const int64_t nd = g.nd;
+  if (nd == 0) return RTG_OK;
+  int64_t nnz = 0;
+  RTG_CUDA(ctx, cudaMemcpyAsync(&nnz, g.nb_ptr.p + nd, sizeof nnz, cudaMemcpyDeviceToHost, st));
+  RTG_CUDA(ctx, cudaStreamSynchronize(st));
+  RTG_TRY(dalloc(ctx, g.nb_idx, (size_t)(nnz > 0 ? nnz : 1), "neighbour columns"));
+  RTG_TRY(dalloc(ctx, g.nb_slot, (size_t)(nnz > 0 ? nnz : 1), "neighbour slots"));
+  g.nb_nnz = nnz;
+  if (nnz == 0) return RTG_OK;
+  Grid grid;
+  for (int a = 0; a < 3; ++a) {
+    grid.org[a] = w.org[a];
+    grid.dim[a] = w.dim[a];
+  }
+  grid.inv_h = w.inv_h;
+  neighbor_kernel<true><<<blocks_for(nd, 128), 128, 0, st>>>(w.cell_disc.p, w.cell_id.p, nd, grid, w.start.p,
+                                                             g.nb_ptr.p, g.disc_slot.p, g.nb_idx.p, g.nb_slot.p);
+  RTG_CUDA(ctx, cudaGetLastError());
+  return RTG_OK;
+}
+
+void release_neighbors(NeighborWork& w, cudaStream_t st) {
+  tfree(w.start, st);
+  tfree(w.cell_rank, st);
+  tfree(w.cell_disc, st);
+  tfree(w.cell_id, st);
 }
 
 int compute_areas_into(rtg_context* ctx, cudaStream_t st, const float* box_lo, const float* box_hi, float* out) {
@@ -446,17 +481,16 @@ int compute_areas(rtg_context* ctx, cudaStream_t st, const float* box_lo, const 
 int finalize_estimates(rtg_context* ctx, cudaStream_t st) {
   Geometry& g = ctx->g;
   const int64_t np = g.nd + g.nt;
-  DBuf<unsigned long long> mx;
-  RTG_TRY(dalloc(ctx, mx, 1, "max"));
-  cudaMemsetAsync(mx.p, 0, sizeof(unsigned long long), st);
-  smooth_kernel<<<blocks_for(np, 256), 256, 0, st>>>(ctx->acc.p, ctx->areas.p, np, g.nd,
-                                                     g.nd > 0 ? g.nb_ptr.p : nullptr, g.nb_idx.p, ctx->est.p,
-                                                     mx.p);
-  divide_kernel<<<blocks_for(np, 256), 256, 0, st>>>(ctx->est.p, np, mx.p);
-  cudaError_t e = cudaStreamSynchronize(st);
-  if (e == cudaSuccess) e = cudaGetLastError();
-  dfree(mx);
-  if (e != cudaSuccess) return check_cuda(ctx, e, "normalised estimates");
+  RTG_TRY(dalloc(ctx, ctx->stat_tmp, (size_t)(2 * np), "estimates"));
+  unsigned long long* mx = reinterpret_cast<unsigned long long*>(ctx->stat_tmp.p);
+  double* flux = ctx->stat_tmp.p + 1;  // at most 2 np - 1 discs
+  RTG_CUDA(ctx, cudaMemsetAsync(mx, 0, sizeof(unsigned long long), st));
+  if (g.nd > 0) flux_kernel<<<blocks_for(g.nd, 256), 256, 0, st>>>(ctx->acc.p, ctx->areas.p, g.nd, flux);
+  smooth_kernel<<<blocks_for(np, 256), 256, 0, st>>>(ctx->acc.p, ctx->areas.p, flux, np, g.nd, g.nb_ptr.p, g.nb_idx.p,
+                                                     ctx->est.p, mx);
+  divide_kernel<<<blocks_for(np, 256), 256, 0, st>>>(ctx->est.p, np, mx);
+  RTG_CUDA(ctx, cudaGetLastError());
+  RTG_CUDA(ctx, cudaStreamSynchronize(st));
   return RTG_OK;
 }
 
