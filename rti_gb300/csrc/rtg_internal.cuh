@@ -34,21 +34,29 @@ struct __align__(16) Node {
 
 // One node as the closest-hit query visits it: up to four boxes below a binary
 // node (its children, the larger ones opened; rtg_lbvh.cu) as centre and half
-// extent, 128 B, at the binary node's index.  The pairs are operands of
-// two-wide float instructions: x and y of one child, or z of two.
-//   xy[k] = (centre.x, centre.y, half.x, half.y) of child k
-//   z[j]  = (centre.z of 2j, of 2j + 1, half.z of 2j, of 2j + 1)
-//   ref   = the children's references; a missing child has half extents -1e30
-//           (a box that no ray meets) and a leaf reference
-// The half extents are rounded up and widened by 2^-20 of themselves and 2^-21
-// of the centre, which covers the rounding of the slab test (quad_test in
+// extent, at the binary node's index.  96 bytes, three loads: a divergent load
+// costs the L1 data pipe one wavefront per lane whatever its width, and that
+// pipe bounds a full GPU.
+//   xy[2k], xy[2k + 1], z[k] = centre of child k
+//   half     = the half extents as bfloat16, rounded up, two a word.  High
+//              halves of words 0..5: x and y of child 0, x and y of child 2, z
+//              of children 0 and 1; low halves: x and y of child 1, x and y of
+//              child 3, z of children 2 and 3.  A high half is read as the
+//              float that its whole word is: the low half makes it larger.
+//   ref[k]   = the child's reference; a missing child has half extents -1e30
+//              (a box that no ray meets) and a leaf reference
+//   inner    = children that are inner nodes
+// Pairs of words are operands of two-wide float instructions.  The half
+// extents are widened by 2^-20 of themselves and 2^-21 of the centre before
+// they are rounded, which covers the rounding of the slab test (quad_test in
 // rtg_path.cuh) for rays that start near the box; the test's relative slack
 // covers it far away.
-struct __align__(128) QuadNode {
-  float4 xy[4];
-  float4 z[2];
-  uint4 ref;
-  uint4 info;  // x: inner children
+struct __align__(32) QuadNode {
+  float xy[8];
+  float z[4];
+  uint32_t half[6];
+  uint32_t ref[4];
+  uint32_t inner, unused;
 };
 
 // One node of the compressed 8-wide tree the closest-hit query may traverse

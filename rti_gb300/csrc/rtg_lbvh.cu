@@ -580,19 +580,13 @@ __global__ void refit_kernel(int64_t n, const uint32_t* __restrict__ parent, con
   atomicAdd(&status[kStRefit], 1ull);
 }
 
-// A box as a QuadNode stores it.
-struct QuadBox {
-  float c[3], h[3];
-};
-__device__ __forceinline__ QuadBox quad_box(const float* lo, const float* hi) {
-  QuadBox q;
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    q.c[a] = 0.5f * lo[a] + 0.5f * hi[a];
-    const float e = fmaxf(__fsub_ru(hi[a], q.c[a]), __fsub_ru(q.c[a], lo[a]));
-    q.h[a] = __fadd_ru(__fmul_ru(e, 1.00000096f), __fmul_ru(fabsf(q.c[a]), 0x1p-21f));
-  }
-  return q;
+// Centre and half extent (a bfloat16, rounded up) of [lo, hi] as a QuadNode
+// stores them.
+__device__ __forceinline__ uint32_t quad_extent(float lo, float hi, float& c) {
+  c = 0.5f * lo + 0.5f * hi;
+  const float e = fmaxf(__fsub_ru(hi, c), __fsub_ru(c, lo));
+  const float h = __fadd_ru(__fmul_ru(e, 1.00000096f), __fmul_ru(fabsf(c), 0x1p-21f));
+  return (__float_as_uint(h) + 0xFFFFu) >> 16;
 }
 
 // The QuadNode of every binary node: its two children and, as long as there is
@@ -635,26 +629,30 @@ __global__ void quad_kernel(const Node* __restrict__ nodes, int64_t n_internal, 
     open(ref[best], best, n);
     ++n;
   }
-  QuadBox q[4];
-  uint32_t inner = 0;
-  for (int k = 0; k < 4; ++k) {
-    if (k < n) {
-      q[k] = quad_box(lo[k], hi[k]);
-      if (!(ref[k] & kLeafBit)) inner += 1;
-    } else {
-      ref[k] = kLeafBit;
-      for (int a = 0; a < 3; ++a) {
-        q[k].c[a] = 0.0f;
-        q[k].h[a] = -1e30f;
-      }
-    }
-  }
+  uint32_t h[4][3];
   QuadNode out;
-  for (int k = 0; k < 4; ++k) out.xy[k] = make_float4(q[k].c[0], q[k].c[1], q[k].h[0], q[k].h[1]);
-  out.z[0] = make_float4(q[0].c[2], q[1].c[2], q[0].h[2], q[1].h[2]);
-  out.z[1] = make_float4(q[2].c[2], q[3].c[2], q[2].h[2], q[3].h[2]);
-  out.ref = make_uint4(ref[0], ref[1], ref[2], ref[3]);
-  out.info = make_uint4(inner, 0u, 0u, 0u);
+  out.inner = 0u;
+  out.unused = 0u;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    float c[3] = {0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      h[k][a] = __float_as_uint(-1e30f) >> 16;
+      if (k < n) h[k][a] = quad_extent(lo[k][a], hi[k][a], c[a]);
+    }
+    out.xy[2 * k] = c[0];
+    out.xy[2 * k + 1] = c[1];
+    out.z[k] = c[2];
+    out.ref[k] = k < n ? ref[k] : kLeafBit;
+    if (!(out.ref[k] & kLeafBit)) out.inner += 1u;
+  }
+  out.half[0] = h[0][0] << 16 | h[1][0];
+  out.half[1] = h[0][1] << 16 | h[1][1];
+  out.half[2] = h[2][0] << 16 | h[3][0];
+  out.half[3] = h[2][1] << 16 | h[3][1];
+  out.half[4] = h[0][2] << 16 | h[2][2];
+  out.half[5] = h[1][2] << 16 | h[3][2];
   quads[i] = out;
 }
 
@@ -680,11 +678,12 @@ __global__ void quad_need_kernel(int64_t n, const uint32_t* __restrict__ parent,
     }
     int at = whole ? len - 1 : -1;  // path[at] is the quad to leave; a broken link is the refit's error
     while (at > 0) {
-      const uint4 r = quads[path[at]].ref;
-      const unsigned int inner = quads[path[at]].info.x;
+      const uint32_t* r = quads[path[at]].ref;
+      const unsigned int inner = quads[path[at]].inner;
+      const uint32_t r0 = r[0], r1 = r[1], r2 = r[2], r3 = r[3];
       int next = -1;
       for (int k = at - 1; k >= 0 && k >= at - 3; --k)
-        if (r.x == path[k] || r.y == path[k] || r.z == path[k] || r.w == path[k]) {
+        if (r0 == path[k] || r1 == path[k] || r2 == path[k] || r3 == path[k]) {
           next = k;
           break;
         }

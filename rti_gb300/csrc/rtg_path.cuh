@@ -111,25 +111,29 @@ __device__ __forceinline__ QuadRay quad_ray(const Ray& r) {
   return q;
 }
 
+// The low halves of two words of QuadNode::half as floats.
+__device__ __forceinline__ f2 low_halves(f2 w) {
+  uint32_t a, b;
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(a), "=r"(b) : "l"(w));
+  return pack2(__uint_as_float(a << 16), __uint_as_float(b << 16));
+}
+
 // The four boxes of a node: hit[k] where the ray meets box k within
 // [tmin, tmax], tn[k] where it enters.  18 two-wide FMAs and no minimum or
 // maximum per slab (lo/hi planes take 24 subtractions, 24 multiplications and
-// 24 minima for as many boxes).  The boxes' margins cover the rounding for a
-// ray that starts near them, the factor 1 + 2^-20 (over eight roundings of
-// 2^-24) for one far away, so a box that holds an accepted hit in
-// [tmin, tmax] is never missed.
+// 24 minima for as many boxes).  A box that holds an accepted hit in
+// [tmin, tmax] is never missed: the factor 1 + 2^-20 is over eight roundings of
+// 2^-24 far from the ray's origin, the boxes' margins cover those near it.
 __device__ __forceinline__ void quad_test(const QuadNode* nd, const QuadRay& q, float tmin, float tmax, bool* hit,
                                           float* tn, uint32_t* ref) {
   const char* p = reinterpret_cast<const char*>(nd);
-  f2 c[4], e[4], cz[2], ez[2];
-  load_pairs(p, c[0], e[0], c[1], e[1]);
-  load_pairs(p + 32, c[2], e[2], c[3], e[3]);
-  load_pairs(p + 64, cz[0], ez[0], cz[1], ez[1]);
-  const uint4 r = __ldg(&nd->ref);
-  ref[0] = r.x;
-  ref[1] = r.y;
-  ref[2] = r.z;
-  ref[3] = r.w;
+  f2 c[4], cz[2], h01, h23, hz, r01, r23, unused;
+  load_pairs(p, c[0], c[1], c[2], c[3]);
+  load_pairs(p + 32, cz[0], cz[1], h01, h23);
+  load_pairs(p + 64, hz, r01, r23, unused);
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(ref[0]), "=r"(ref[1]) : "l"(r01));
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(ref[2]), "=r"(ref[3]) : "l"(r23));
+  const f2 e[4] = {h01, low_halves(h01), h23, low_halves(h23)}, ez[2] = {hz, low_halves(hz)};
   float nz[4], fz[4];
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
@@ -307,14 +311,17 @@ __device__ __forceinline__ bool closest_hit_wide(const SceneView& s, const Ray& 
 
 // Closest primitive hit; returns false when nothing is hit.  errs counts
 // stack overflows and visit-limit trips (both end the query).
-// Bound by instructions at low SIMD efficiency (6 of 32 lanes on the hole: the
-// lanes wait for the longest query of their warp, leaf tests run for two lanes
-// at a time) and by the chain of dependent loads and instructions in the tail.
-// Up to four boxes a visit (QuadNode): half the dependent loads of a visit per
-// binary node, and about the same instructions.  One launch, before (binary
-// nodes, lo/hi planes) and now: trench 1e6 rays 3.13 -> 2.23 ms, hole (200 k
-// triangles) 1e6 rays 17.7 -> 13.8 and 1e7 rays 52.2 -> 47.2, 2e7 rays onto
-// 4.19 M discs 30.5 (8-wide tree) -> 27.6.
+// Up to four boxes a visit (QuadNode).  A full GPU is bound by what a visit
+// issues (70 % of the slots, the ALU pipe at 56 %) and by the L1 data pipe (one
+// wavefront per lane and load, 53 %); a launch's tail by the chain of a single
+// path's instructions and loads.  The lanes wait for the longest query of their
+// warp, and leaf tests run for two lanes at a time.  One launch over the binary
+// nodes (two boxes and two loads a visit, lo/hi planes), over 128-byte quads
+// (four loads), over these (three): trench 1e6 rays 3.13, 2.23, 2.19 ms; hole
+// (200 k triangles) 1e6 rays 17.7, 13.8, 13.8 and 1e7 rays 52.2, 46.9, 44.1; 2e7
+// rays onto 4.19 M discs 30.5 (8-wide tree), 27.6, 25.8.  64-byte quads (two
+// loads, 16-bit centres in a frame of the surface) cost 12 to 24 byte permutes a
+// visit and wider boxes: 2.35, 14.4, 46.6, 25.5.
 // Boxes that the ray leaves before tnear are skipped, since a hit
 // needs t > tnear: a ray that starts on a flat face passes over the whole face.
 // Leaf children hit are tested on the spot; of the inner ones the nearest is
