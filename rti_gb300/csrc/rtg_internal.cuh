@@ -149,6 +149,7 @@ struct TraceParams {
   uint32_t max_segments;
   uint32_t job;
   int32_t packet;  // a warp takes new source rays when at least this many lanes are idle
+  int32_t lanes;   // paths a warp holds at most (32 in a plain launch)
   int32_t plain;   // 1: one source ray per thread, no refill (grid covers all rays)
   int32_t fixed_s1;       // 1: s1 holds int64 multiples of 2^-32 during the trace (RTG_ACCUM_FIXED)
   int32_t window;         // 1: multi-hit window deposit (RTG_DEPOSIT_WINDOW), traced by kModeWindow
@@ -332,6 +333,8 @@ bool use_wide(const rtg_context* ctx);
 // the traversal stack depth a query of ctx can need (binary tree depth, or
 // the wide tree's stack need when it is used)
 int traversal_depth(const rtg_context* ctx);
+// sets the paths a warp holds in a launch of nrays; returns the blocks of tpb threads that hold all
+uint64_t spread_rays(TraceParams& p, uint64_t nrays, int tpb, int sms);
 // stack entries for a requested depth (0 = automatic) and a tree depth: 32, 64 or 256
 int stack_for(int requested, int tree_depth);
 // RTG_ACCUM_FIXED: s1 between double and int64 multiples of 2^-32, in place

@@ -9,7 +9,8 @@
 // diffuse/specular re-emission.  Threads are persistent: when at
 // least `packet` lanes of a warp are idle, the warp takes that many next
 // source-ray ids from a global counter (one atomic per warp), so long and
-// short paths share the SIMD lanes.
+// short paths share the SIMD lanes.  In a launch of fewer rays than the GPU has
+// lanes for, a warp's share is `lanes` paths instead of 32.
 //
 // Closest hit = stack traversal of the tree's four-box nodes; ties in t go to
 // the lower primitive id, and the node boxes are conservative, so the chosen
@@ -731,20 +732,22 @@ __global__ void __launch_bounds__(TPB, resident_threads(M) / TPB)
   for (uint32_t iter = 0;; ++iter) {
     if (!exhausted) {
       const unsigned need = __ballot_sync(kFull, !active);
-      if (need && __popc(need) >= p0.packet) {
+      const int take = __popc(need) - 32 + p0.lanes;  // what is left of the warp's share of paths
+      if (take > 0 && take >= p0.packet) {
         const int leader = __ffs(need) - 1;
         unsigned long long base = 0;
         if (p0.plain) {  // one source ray per thread (all lanes are idle on the first pass)
           base = (unsigned long long)blockIdx.x * TPB + (threadIdx.x & ~31u);
           exhausted = true;
         } else {
-          if (lane == leader) base = atomicAdd(&p0.tally->next_ray, (unsigned long long)__popc(need));
+          if (lane == leader) base = atomicAdd(&p0.tally->next_ray, (unsigned long long)take);
           base = __shfl_sync(kFull, base, leader);
-          if (base + __popc(need) >= nrays) exhausted = true;
+          if (base + take >= nrays) exhausted = true;
         }
         if (!active) {
-          const uint64_t j = base + (uint64_t)__popc(need & lt_mask);
-          if (j < nrays) {
+          const int r = __popc(need & lt_mask);
+          const uint64_t j = base + (uint64_t)r;
+          if (r < take && j < nrays) {
             if (Batched) {
               int lo = 0, hi = njobs - 1;  // last job whose first id <= j
               while (lo < hi) {

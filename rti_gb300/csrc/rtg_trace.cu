@@ -123,6 +123,24 @@ int stack_for(int requested, int tree_depth) {
   return 256;
 }
 
+// Sets the paths that each warp holds (p.lanes) for a launch of nrays and
+// returns the blocks of tpb threads that hold them all.  A warp's time per
+// segment grows with the paths in it, since they part ways: alone a path takes
+// a third of what 32 take together.  So a launch that the GPU could hold at
+// once is spread over 16 warps an SM before any warp gets more.  Packed warps
+// -> 8, 16, 24, 32 warps an SM: 1024 rays into a trench of 1500 discs 266 -> 174,
+// 176, 177, 176 us; 16 384 into one of 98 k discs 698 -> 606, 546, 657, 557; 50 000
+// onto 4.19 M discs 323 -> 321, 311, 315, 335; from 78 000 rays on (32 paths a
+// warp) nothing changes.
+uint64_t spread_rays(TraceParams& p, uint64_t nrays, int tpb, int sms) {
+  const uint64_t warps = 16 * (uint64_t)sms;
+  const uint64_t share = std::max<uint64_t>(1, nrays / warps + (nrays % warps != 0));
+  p.lanes = p.plain ? 32 : (int)std::min<uint64_t>(32, share);
+  p.packet = std::min(p.packet, p.lanes);
+  const uint64_t held = (uint64_t)(tpb / 32) * p.lanes;
+  return std::max<uint64_t>(1, nrays / held + (nrays % held != 0));
+}
+
 int check_launch_config(rtg_context* ctx, const rtg_launch_config& lc) {
   auto bad = [&](const char* m) { return set_error(ctx, RTG_ERR_INVALID_ARGUMENT, m); };
   if (lc.threads_per_block != 64 && lc.threads_per_block != 128 && lc.threads_per_block != 256)
@@ -201,8 +219,8 @@ int launch_trace(rtg_context* ctx, const TraceParams& p_in, cudaStream_t st, int
   RTG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, tpb, 0));
   if (per_sm < 1) per_sm = 1;
   uint64_t blocks = (uint64_t)sms * per_sm;
-  const uint64_t full = (nrays + tpb - 1) / tpb;
-  if (full < blocks || p.plain) blocks = full > 0 ? full : 1;
+  const uint64_t full = spread_rays(p, nrays, tpb, sms);
+  if (full < blocks || p.plain) blocks = full;
   if (blocks > 0x7FFFFFFFull) return set_error(ctx, RTG_ERR_INVALID_ARGUMENT, "too many rays for a plain launch");
   kern<<<(unsigned)blocks, tpb, 0, st>>>(p, nullptr, nullptr, 0);
   RTG_CUDA(ctx, cudaGetLastError());

@@ -34,8 +34,8 @@ int launch_trace_batched(rtg_context* ctx, const TraceParams& p0_in, const Trace
   RTG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, tpb, 0));
   if (per_sm < 1) per_sm = 1;
   uint64_t blocks = (uint64_t)sms * per_sm;
-  const uint64_t need = (total_rays + tpb - 1) / tpb;
-  if (need < blocks || p0.plain) blocks = need > 0 ? need : 1;
+  const uint64_t need = spread_rays(p0, total_rays, tpb, sms);
+  if (need < blocks || p0.plain) blocks = need;
   if (blocks > 0x7FFFFFFFull) return set_error(ctx, RTG_ERR_INVALID_ARGUMENT, "too many rays for a plain launch");
   kern<<<(unsigned)blocks, tpb, 0, st>>>(p0, d_jobs, d_prefix, njobs);
   RTG_CUDA(ctx, cudaGetLastError());
