@@ -198,8 +198,8 @@ int launch_trace(rtg_context* ctx, const TraceParams& p_in, cudaStream_t st, int
   // so has a trace that fills the segment log
   if (mode == kModeForward && p.window) mode = kModeWindow;
   if (mode == kModeForward && p.log.rec) mode = kModeLogged;
-  // the window's interval queries walk the binary tree
-  const int need = mode == kModeWindow ? std::max(ctx->g.depth, traversal_depth(ctx)) : traversal_depth(ctx);
+  // the window's interval queries visit the quads, whichever tree the closest hits use
+  const int need = mode == kModeWindow ? std::max(ctx->g.quad_stack, traversal_depth(ctx)) : traversal_depth(ctx);
   const int stack = stack_for(lc.stack_depth, need);
   if (mode == kModeForward && lc.scheduling == RTG_SCHED_WAVEFRONT) {
     // a job table of one entry
