@@ -249,6 +249,7 @@ struct rtg_context {
   rtg::DBuf<unsigned char> scratch;
   size_t scratch_top = 0;
   bool scratch_open = false;
+  rtg::DBuf<unsigned char> queries;  // rtg_trace_rays: rays and results of a call, at most kScratchMax kept
   // segment log (rtg_set_segment_log)
   rtg::DBuf<rtg_segment> seglog;
   rtg::DBuf<unsigned long long> seglog_count;

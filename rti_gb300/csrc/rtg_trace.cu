@@ -8,24 +8,34 @@ namespace rtg {
 
 namespace {
 
-__global__ void closest_hit_kernel(const SceneView s, const float* __restrict__ rays, int64_t n, float tnear,
-                                   int32_t* __restrict__ prim, float* __restrict__ tout,
-                                   unsigned long long* errors) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+constexpr int kQueryThreads = 128;
+
+// Closest hits of explicit rays, `share` of them a warp, bound as a trace's
+// queries are.  The stack follows the tree's need (a 256-entry one in every
+// thread and the wide traversal compiled in went with 230 us more a call).
+// Whole calls of 262 144 rays, before -> now: hole of 31 k triangles 479 -> 219 us,
+// trench of 98 k discs 488 -> 198, 4.19 M discs 707 -> 379; 1000 rays 106 -> 81.
+// 768, 1280 and 1536 threads an SM: 230, 224, 245 us for the hole.
+template <int STACK, bool WIDE>
+__global__ void __launch_bounds__(kQueryThreads, 1024 / kQueryThreads)
+    closest_hit_kernel(const SceneView s, const float* __restrict__ rays, int64_t n, int share, float tnear,
+                       int32_t* __restrict__ prim, float* __restrict__ tout, unsigned long long* errors) {
+  const int lane = threadIdx.x & 31;
+  const int64_t i = ((int64_t)blockIdx.x * (kQueryThreads / 32) + threadIdx.x / 32) * share + lane;
+  if (lane >= share || i >= n) return;
   const float* r = rays + 6 * i;
   float t;
   int id;
   uint32_t ref;
-  unsigned long long e = 0;
-  if (closest_hit<256>(s, mk3(r[0], r[1], r[2]), mk3(r[3], r[4], r[5]), tnear, t, id, ref, e)) {
+  uint32_t e = 0;
+  if (closest_hit<STACK, 0, WIDE>(s, mk3(r[0], r[1], r[2]), mk3(r[3], r[4], r[5]), tnear, t, id, ref, e)) {
     prim[i] = id;
     tout[i] = t;
   } else {
     prim[i] = -1;
     tout[i] = 0.0f;
   }
-  if (e) atomicAdd(errors, e);
+  if (e) atomicAdd(errors, (unsigned long long)e);
 }
 
 template <int TPB>
@@ -123,8 +133,7 @@ int stack_for(int requested, int tree_depth) {
   return 256;
 }
 
-// Sets the paths that each warp holds (p.lanes) for a launch of nrays and
-// returns the blocks of tpb threads that hold them all.  A warp's time per
+// The paths that each warp holds in a launch of nrays.  A warp's time per
 // segment grows with the paths in it, since they part ways: alone a path takes
 // a third of what 32 take together.  So a launch that the GPU could hold at
 // once is spread over 16 warps an SM before any warp gets more.  Packed warps
@@ -132,10 +141,13 @@ int stack_for(int requested, int tree_depth) {
 // 176, 177, 176 us; 16 384 into one of 98 k discs 698 -> 606, 546, 657, 557; 50 000
 // onto 4.19 M discs 323 -> 321, 311, 315, 335; from 78 000 rays on (32 paths a
 // warp) nothing changes.
-uint64_t spread_rays(TraceParams& p, uint64_t nrays, int tpb, int sms) {
+int warp_share(uint64_t nrays, int sms) {
   const uint64_t warps = 16 * (uint64_t)sms;
-  const uint64_t share = std::max<uint64_t>(1, nrays / warps + (nrays % warps != 0));
-  p.lanes = p.plain ? 32 : (int)std::min<uint64_t>(32, share);
+  return (int)std::min<uint64_t>(32, std::max<uint64_t>(1, nrays / warps + (nrays % warps != 0)));
+}
+
+uint64_t spread_rays(TraceParams& p, uint64_t nrays, int tpb, int sms) {
+  p.lanes = p.plain ? 32 : warp_share(nrays, sms);
   p.packet = std::min(p.packet, p.lanes);
   const uint64_t held = (uint64_t)(tpb / 32) * p.lanes;
   return std::max<uint64_t>(1, nrays / held + (nrays % held != 0));
@@ -231,8 +243,18 @@ int launch_closest_hit(rtg_context* ctx, const float* d_rays, int64_t n, float t
                        unsigned long long* d_errors, cudaStream_t st) {
   if (n <= 0) return RTG_OK;
   RTG_TRY(ensure_wide(ctx));
-  SceneView s = scene_view(ctx);
-  closest_hit_kernel<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(s, d_rays, n, tnear, d_prim, d_t, d_errors);
+  const SceneView s = scene_view(ctx);
+  const int stack = stack_for(0, traversal_depth(ctx));
+  int sms = 0;
+  RTG_CUDA(ctx, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
+  const int share = warp_share((uint64_t)n, sms);
+  const int64_t held = (int64_t)(kQueryThreads / 32) * share, blocks = (n + held - 1) / held;
+  if (blocks > 0x7FFFFFFFll) return set_error(ctx, RTG_ERR_INVALID_ARGUMENT, "too many rays for one launch");
+  auto kern = s.wnodes ? closest_hit_kernel<256, true>
+              : stack <= 32 ? closest_hit_kernel<32, false>
+              : stack <= 64 ? closest_hit_kernel<64, false>
+                            : closest_hit_kernel<256, false>;
+  kern<<<(unsigned)blocks, kQueryThreads, 0, st>>>(s, d_rays, n, share, tnear, d_prim, d_t, d_errors);
   RTG_CUDA(ctx, cudaGetLastError());
   return RTG_OK;
 }
