@@ -618,6 +618,7 @@ int rtg_destroy(rtg_context* ctx) {
   dfree(ctx->stat_tmp);
   dfree(ctx->scratch);
   dfree(ctx->queries);
+  for (auto& b : ctx->ray_order) dfree(b);
   dfree(g.wnodes);
   dfree(ctx->seglog);
   dfree(ctx->seglog_count);

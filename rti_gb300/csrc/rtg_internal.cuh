@@ -150,6 +150,7 @@ struct TraceParams {
   uint32_t job;
   int32_t packet;  // a warp takes new source rays when at least this many lanes are idle
   int32_t lanes;   // paths a warp holds at most (32 in a plain launch)
+  const uint32_t* order;  // ray ids less ray_begin in the order they are taken, or nullptr: ascending
   int32_t plain;   // 1: one source ray per thread, no refill (grid covers all rays)
   int32_t fixed_s1;       // 1: s1 holds int64 multiples of 2^-32 during the trace (RTG_ACCUM_FIXED)
   int32_t window;         // 1: multi-hit window deposit (RTG_DEPOSIT_WINDOW), traced by kModeWindow
@@ -249,6 +250,7 @@ struct rtg_context {
   rtg::DBuf<unsigned char> scratch;
   size_t scratch_top = 0;
   bool scratch_open = false;
+  rtg::DBuf<uint32_t> ray_order[2];  // cells | ray ids of an ordered launch (trace, adjoint), kept; see launch_trace
   rtg::DBuf<unsigned char> queries;  // rtg_trace_rays: rays and results of a call, at most kScratchMax kept
   // segment log (rtg_set_segment_log)
   rtg::DBuf<rtg_segment> seglog;

@@ -762,7 +762,7 @@ __global__ void __launch_bounds__(TPB, resident_threads(M) / TPB)
               pp = jobs + lo;
               id = pp->ray_begin + (j - __ldg(&prefix[lo]));
             } else {
-              id = p0.ray_begin + j;
+              id = p0.ray_begin + (p0.order ? (uint64_t)__ldg(&p0.order[j]) : j);
             }
             // source.hpp:20-58 with rectangle_origin_z / (power_)cosine_direction_z
             const uint4 u = draw4(pp->seed, id, 0xFFFFFFFFu, pp->job);

@@ -38,6 +38,35 @@ __global__ void __launch_bounds__(kQueryThreads, 1024 / kQueryThreads)
   if (e) atomicAdd(errors, (unsigned long long)e);
 }
 
+// Ordered launches: a counting sort of the rays by the cell that they start in,
+// so that a warp's paths, and those in flight around them, visit the same
+// nodes.  A cell is one of 64 x 64 parts of the source rectangle (in Morton order)
+// and a quarter turn of the direction, all of them high bits of the source draw.
+constexpr int kCellBits = 6, kTurnBits = 2, kCells = 1 << (2 * kCellBits + kTurnBits);
+constexpr uint64_t kOrderMax = 1u << 25;  // rays ordered at once (128 MB of ids)
+
+__device__ __forceinline__ uint32_t spread_bits(uint32_t v) {  // 6 bits to every second place
+  v = (v | v << 4) & 0x0F0Fu;
+  v = (v | v << 2) & 0x3333u;
+  return (v | v << 1) & 0x5555u;
+}
+__device__ __forceinline__ uint32_t source_cell(const TraceParams& p, uint32_t j) {
+  const uint4 u = draw4(p.seed, p.ray_begin + j, 0xFFFFFFFFu, p.job);
+  const uint32_t place = spread_bits(u.x >> (32 - kCellBits)) << 1 | spread_bits(u.y >> (32 - kCellBits));
+  return place << kTurnBits | u.z >> (32 - kTurnBits);
+}
+// One thread per ray, bound by the atomics on the cells (2e7 rays: 0.12 ms to
+// count, 0.23 ms to place; the trace of these takes 13 to 16 ms).
+__global__ void order_count_kernel(const __grid_constant__ TraceParams p, uint32_t n, uint32_t* __restrict__ cells) {
+  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j < n) atomicAdd(&cells[source_cell(p, j)], 1u);
+}
+__global__ void order_place_kernel(const __grid_constant__ TraceParams p, uint32_t n, uint32_t* __restrict__ cells,
+                                   uint32_t* __restrict__ order) {
+  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j < n) order[atomicAdd(&cells[source_cell(p, j)], 1u)] = j;
+}
+
 template <int TPB>
 PathKernel forward_kernel(int stack, bool shared, bool wide) {
   if (stack <= 32) return kernel_for<kModeForward, false, TPB, 32>(shared, wide);
@@ -201,6 +230,49 @@ SceneView scene_view(rtg_context* ctx) {
   return s;
 }
 
+namespace {
+
+// Whether a launch takes its rays by the cells they start in.  It does where
+// paths that start together share memory that others would evict, on a surface
+// that outgrows the L2 cache, and where they stay together for long, in a surface
+// as deep as it is wide; on a flat surface that the cache holds they only meet in
+// their deposits.  Ascending ids -> ordered, launch and sort, in us:
+//   4.19 M discs                1e6 rays 1226 -> 1123, 4e6 4279 -> 3515, 1.6e7 16540 -> 12998
+//   their field adjoint         5e6 rays 5940 -> 4840
+//   directional, disc hole      1e6 rays 995 -> 907, 2e6 1624 -> 1412, 4e6 3031 -> 2405, 1.6e7 11329 -> 8668
+//   trench                      1e6 rays 2048 -> 2070, 2e6 3215 -> 3239, 4e6 5600 -> 5415, 1.6e7 19640 -> 19140
+//   hole, 200 k triangles       1e6 rays the same, 4e6 23200 -> 22830, 1.6e7 63170 -> 61080
+//   flat, 262 k discs           1e6 rays 790 -> 818, 4e6 2708 -> 2789, 1.6e7 10979 -> 11284: not ordered
+bool wants_order(const rtg_context* ctx, const TraceParams& p, uint64_t nrays) {
+  if (nrays < 1u << 20) return false;
+  if (outgrows_l2(ctx)) return true;
+  const float wide = std::max(p.box_hi[0] - p.box_lo[0], p.box_hi[1] - p.box_lo[1]);
+  return nrays >= 1u << 21 && p.box_hi[2] - p.box_lo[2] >= wide;
+}
+
+// Room for the cells and the ids of an ordered launch, kept by the context (at
+// most 128 MB).  Without it, or while the stream is being captured (the buffer may
+// be another one when the graph runs), the launch takes its rays in ascending order.
+bool room_for_order(rtg_context* ctx, DBuf<uint32_t>& ids, cudaStream_t st, uint64_t rays) {
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return false;
+  }
+  const size_t words = kCells + (size_t)rays;
+  if (ids.n >= words) return true;
+  dfree(ids);
+  if (injected_alloc_failure(ctx) || cudaMalloc((void**)&ids.p, words * sizeof(uint32_t)) != cudaSuccess) {
+    cudaGetLastError();
+    ids.p = nullptr;
+    return false;
+  }
+  ids.n = words;
+  return true;
+}
+
+}  // namespace
+
 int launch_trace(rtg_context* ctx, const TraceParams& p_in, cudaStream_t st, int mode) {
   const rtg_launch_config& lc = ctx->lc;
   TraceParams p = p_in;
@@ -230,12 +302,40 @@ int launch_trace(rtg_context* ctx, const TraceParams& p_in, cudaStream_t st, int
   RTG_CUDA(ctx, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
   RTG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, tpb, 0));
   if (per_sm < 1) per_sm = 1;
-  uint64_t blocks = (uint64_t)sms * per_sm;
-  const uint64_t full = spread_rays(p, nrays, tpb, sms);
-  if (full < blocks || p.plain) blocks = full;
-  if (blocks > 0x7FFFFFFFull) return set_error(ctx, RTG_ERR_INVALID_ARGUMENT, "too many rays for a plain launch");
-  kern<<<(unsigned)blocks, tpb, 0, st>>>(p, nullptr, nullptr, 0);
-  RTG_CUDA(ctx, cudaGetLastError());
+  // one launch, or several of ordered rays
+  uint64_t chunk = nrays;
+  DBuf<uint32_t>& ids = ctx->ray_order[mode == kModeAdjGlobal || mode == kModeAdjField ? 1 : 0];
+  bool ordered = mode != kModeLogged && wants_order(ctx, p, nrays);
+  if (ordered) {
+    const uint64_t chunks = (nrays + kOrderMax - 1) / kOrderMax;
+    chunk = (nrays + chunks - 1) / chunks;
+    ordered = room_for_order(ctx, ids, st, chunk);
+    if (!ordered) chunk = nrays;
+  }
+  const uint64_t end = p.ray_end;
+  for (uint64_t begin = p.ray_begin; begin < end; begin += chunk) {
+    p.ray_begin = begin;
+    p.ray_end = std::min(end, begin + chunk);
+    const uint64_t n = p.ray_end - p.ray_begin;
+    if (ordered) {
+      const unsigned grid = (unsigned)((n + 255) / 256);
+      uint32_t* cells = ids.p;
+      p.order = ids.p + kCells;
+      RTG_CUDA(ctx, cudaMemsetAsync(cells, 0, kCells * sizeof(uint32_t), st));
+      order_count_kernel<<<grid, 256, 0, st>>>(p, (uint32_t)n, cells);
+      RTG_TRY(exclusive_scan_u32(ctx, cells, kCells, nullptr, st));
+      order_place_kernel<<<grid, 256, 0, st>>>(p, (uint32_t)n, cells, ids.p + kCells);
+    }
+    if (begin != p_in.ray_begin)
+      RTG_CUDA(ctx, cudaMemsetAsync(&p.tally->next_ray, 0, sizeof(unsigned long long), st));
+    uint64_t blocks = (uint64_t)sms * per_sm;
+    const uint64_t full = spread_rays(p, n, tpb, sms);
+    if (full < blocks || p.plain) blocks = full;
+    if (blocks > 0x7FFFFFFFull) return set_error(ctx, RTG_ERR_INVALID_ARGUMENT, "too many rays for a plain launch");
+    kern<<<(unsigned)blocks, tpb, 0, st>>>(p, nullptr, nullptr, 0);
+    RTG_CUDA(ctx, cudaGetLastError());
+    if (end - begin <= chunk) break;  // begin + chunk may pass 2^64
+  }
   return RTG_OK;
 }
 
