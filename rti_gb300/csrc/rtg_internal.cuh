@@ -99,6 +99,7 @@ struct SceneView {
   // triangles in slot order, 64 B each: (v0, original id bits), e1, e2, unit normal
   const float4* tri;
   int32_t nt;
+  const float4* basis;  // by slot, discs then triangles, 32 B each: the basis of the normal (pack_basis)
   const Node* nodes;       // the binary tree (the window deposit's interval queries)
   const QuadNode* quads;   // the same tree as closest hits visit it, up to four boxes a node
   uint32_t root;        // child reference of the root (internal node 0 or a leaf)
@@ -189,6 +190,7 @@ struct Geometry {
   // slot-ordered copies
   DBuf<float4> disc;       // 2 per slot: (centre, radius), (normal, id bits)
   DBuf<float4> tri;        // 4 per slot: (v0, id bits), e1, e2, unit normal
+  DBuf<float4> basis;      // 2 per slot, discs then triangles (pack_basis)
   DBuf<Node> nodes;
   DBuf<QuadNode> quads;
   DBuf<uint32_t> leaf_ref;    // per sorted leaf i: child reference

@@ -158,7 +158,7 @@ __global__ void slots_kernel(const uint32_t* __restrict__ sorted_prim, const uin
                              const float4* __restrict__ dn_id, const float4* __restrict__ tv,
                              const uint32_t* __restrict__ tidx, float4* __restrict__ disc,
                              uint32_t* __restrict__ disc_slot, float4* __restrict__ tri,
-                             uint32_t* __restrict__ leaf_ref, int32_t* __restrict__ leaf_prim) {
+                             uint32_t* __restrict__ leaf_ref, int32_t* __restrict__ leaf_prim, float4* __restrict__ basis) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= np) return;
   const uint32_t p = min(sorted_prim[i], (uint32_t)(np - 1));  // a failed sort (reported) leaves anything here
@@ -171,6 +171,8 @@ __global__ void slots_kernel(const uint32_t* __restrict__ sorted_prim, const uin
     disc_slot[p] = ds;
     disc[2 * (int64_t)ds + 1] = make_float4(n.x, n.y, n.z, __int_as_float((int)p));
     leaf_ref[i] = kLeafBit | ds;
+    const f3 nv = mk3(n.x, n.y, n.z);
+    pack_basis(normal_basis(nv), nv, basis[2 * (int64_t)ds], basis[2 * (int64_t)ds + 1]);
   } else {
     uint32_t ts = (uint32_t)i - ds;
     int64_t t = (int64_t)p - nd;
@@ -185,6 +187,7 @@ __global__ void slots_kernel(const uint32_t* __restrict__ sorted_prim, const uin
     tri[4 * (int64_t)ts + 2] = make_float4(e2.x, e2.y, e2.z, 0.0f);
     tri[4 * (int64_t)ts + 3] = make_float4(n.x, n.y, n.z, 0.0f);
     leaf_ref[i] = kLeafBit | kTriBit | ts;
+    pack_basis(normal_basis(n), n, basis[2 * (nd + ts)], basis[2 * (nd + ts) + 1]);
   }
 }
 
@@ -887,7 +890,7 @@ int run_slots(rtg_context* ctx, const uint32_t* d_sorted_prim, cudaStream_t st) 
   }
   slots_kernel<<<blocks_for(np, 256), 256, 0, st>>>(d_sorted_prim, rank.p, np, g.nd, g.disc_cr_by_id.p,
                                                     g.disc_n_by_id.p, g.tri_v.p, g.tri_idx.p, g.disc.p, g.disc_slot.p,
-                                                    g.tri.p, g.leaf_ref.p, g.leaf_prim.p);
+                                                    g.tri.p, g.leaf_ref.p, g.leaf_prim.p, g.basis.p);
   tfree(rank, st);
   RTG_CUDA(ctx, cudaGetLastError());
   return RTG_OK;
@@ -982,6 +985,7 @@ int build_lbvh(rtg_context* ctx) {
     if ((rc = dalloc(ctx, g.disc, (size_t)(2 * (g.nd ? g.nd : 1)), "disc slots")) != RTG_OK) break;
     if ((rc = dalloc(ctx, g.disc_slot, (size_t)(g.nd ? g.nd : 1), "disc slot map")) != RTG_OK) break;
     if ((rc = dalloc(ctx, g.tri, (size_t)(4 * (g.nt ? g.nt : 1)), "triangle slots")) != RTG_OK) break;
+    if ((rc = dalloc(ctx, g.basis, (size_t)(2 * np), "normal bases")) != RTG_OK) break;
     if ((rc = dalloc(ctx, g.leaf_ref, (size_t)np, "leaf references")) != RTG_OK) break;
     if ((rc = dalloc(ctx, g.leaf_prim, (size_t)np, "leaf primitives")) != RTG_OK) break;
     const int64_t nn = np > 1 ? np - 1 : 1;

@@ -169,30 +169,57 @@ __device__ __forceinline__ f3 source_dir(float expo, float ee, uint32_t u_phi, u
   return normalize3(mk3(cs * sq, sn * sq, zz));
 }
 
-// util::get_orthonormal_basis (utils.hpp:207-244) + cos_hemi::get (cos_hemi.hpp:11-45)
-__device__ __forceinline__ f3 diffuse_dir(f3 n, uint32_t u_phi, uint32_t u_t) {
-  f3 c0 = mk3(n.z, n.z, -(n.x + n.y));
-  f3 c1 = mk3(n.y, -(n.x + n.z), n.y);
-  f3 c2 = mk3(-(n.y + n.z), n.x, n.x);
-  f3 b1 = c0;
+// util::get_orthonormal_basis (utils.hpp:207-244): b0 along n, b1 from the one
+// of three vectors with two equal components whose components add up to most.
+struct Basis {
+  f3 b0, b1, b2;
+};
+__device__ __forceinline__ int tangent_case(f3 n) {
+  const f3 c0 = mk3(n.z, n.z, -(n.x + n.y)), c1 = mk3(n.y, -(n.x + n.z), n.y), c2 = mk3(-(n.y + n.z), n.x, n.x);
+  int k = 0;
   float best = c0.x + c0.y + c0.z;
   if (c1.x + c1.y + c1.z > best) {
-    b1 = c1;
+    k = 1;
     best = c1.x + c1.y + c1.z;
   }
-  if (c2.x + c2.y + c2.z > best) b1 = c2;
-  f3 b2 = cross3(n, b1);
-  f3 b0 = normalize3(n);
-  b1 = normalize3(b1);
-  b2 = normalize3(b2);
+  if (c2.x + c2.y + c2.z > best) k = 2;
+  return k;
+}
+__device__ __forceinline__ Basis normal_basis(f3 n) {
+  const int k = tangent_case(n);
+  Basis b;
+  b.b1 = k == 0   ? mk3(n.z, n.z, -(n.x + n.y))
+         : k == 1 ? mk3(n.y, -(n.x + n.z), n.y)
+                  : mk3(-(n.y + n.z), n.x, n.x);
+  b.b2 = normalize3(cross3(n, b.b1));
+  b.b0 = normalize3(n);
+  b.b1 = normalize3(b.b1);
+  return b;
+}
+
+// The basis of a primitive's normal as a scene keeps it, 32 bytes a primitive:
+// b0 | the equal components of b1, b2 | the other component of b1 (quotients of
+// equal operands are equal, and which component is the other one follows from n).
+__device__ __forceinline__ void pack_basis(const Basis& b, f3 n, float4& p, float4& q) {
+  const int k = tangent_case(n);
+  p = make_float4(b.b0.x, b.b0.y, b.b0.z, k == 2 ? b.b1.y : b.b1.x);
+  q = make_float4(b.b2.x, b.b2.y, b.b2.z, k == 0 ? b.b1.z : k == 1 ? b.b1.y : b.b1.x);
+}
+__device__ __forceinline__ Basis unpack_basis(float4 p, float4 q, f3 n) {
+  const int k = tangent_case(n);
+  return Basis{mk3(p.x, p.y, p.z), mk3(k == 2 ? q.w : p.w, k == 1 ? q.w : p.w, k == 0 ? q.w : p.w), mk3(q.x, q.y, q.z)};
+}
+
+// cos_hemi::get (cos_hemi.hpp:11-45)
+__device__ __forceinline__ f3 diffuse_dir(const Basis& b, uint32_t u_phi, uint32_t u_t) {
   float r2 = u01_oc(u_t);
   float cc1 = sqrtf(r2);
   float sq = sqrtf(1.0f - r2);
   float sn, cs;
   sincos2pi(u01_co(u_phi), sn, cs);
   float cc2 = cs * sq, cc3 = sn * sq;
-  return mk3(b0.x * cc1 + b1.x * cc2 + b2.x * cc3, b0.y * cc1 + b1.y * cc2 + b2.y * cc3,
-             b0.z * cc1 + b1.z * cc2 + b2.z * cc3);
+  return mk3(b.b0.x * cc1 + b.b1.x * cc2 + b.b2.x * cc3, b.b0.y * cc1 + b.b1.y * cc2 + b.b2.y * cc3,
+             b.b0.z * cc1 + b.b1.z * cc2 + b.b2.z * cc3);
 }
 
 // specular::use (specular.hpp:66-90): d' = n * (2 n.(-d)) + d

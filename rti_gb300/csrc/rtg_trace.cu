@@ -220,6 +220,7 @@ SceneView scene_view(rtg_context* ctx) {
   s.nt = (int32_t)g.nt;
   s.nodes = g.nodes.p;
   s.quads = g.quads.p;
+  s.basis = g.basis.p;
   s.root = g.root;
   s.nb_ptr = g.nd > 0 ? g.nb_ptr.p : nullptr;
   s.nb_slot = g.nb_slot.p;

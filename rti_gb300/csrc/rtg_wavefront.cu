@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(TPB) wf_shade_kernel(const TraceParams* __rest
             const bool spec = pp->reflection == RTG_REFLECT_SPECULAR ||
                               (pp->reflection == RTG_REFLECT_MIXED &&
                                (double)u.w < (double)pp->specular_fraction * 4294967296.0);
-            d = spec ? specular_dir(nv, d) : diffuse_dir(nv, u.y, u.z);
+            d = spec ? specular_dir(nv, d) : diffuse_dir(normal_basis(nv), u.y, u.z);
             o = hp;
             k += 1;
             cont = true;
