@@ -63,14 +63,36 @@ void drop_graph(rtg_batch* b) {
   b->graph = nullptr;
 }
 
+// The jobs in the order in which the launch takes their rays: those of long paths
+// first (low sticking, a field of it counting as such, then a deep surface): the
+// longest ones, begun last, would run on alone.  Six surfaces, three species, 3.6e6
+// rays, as added -> this: 14.2 -> 12.8 ms; depth first, or by the collisions that
+// both allow: the same.
+std::vector<int> launch_order(const rtg_batch* b) {
+  std::vector<int> order(b->jobs.size());
+  for (size_t i = 0; i < order.size(); ++i) order[i] = (int)i;
+  auto depth = [](const TraceParams& p) {
+    return (double)(p.box_hi[2] - p.box_lo[2]) / std::max(p.box_hi[0] - p.box_lo[0], p.box_hi[1] - p.box_lo[1]);
+  };
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
+    const TraceParams &p = b->jobs[x].p, &q = b->jobs[y].p;
+    const float ps = p.s.sticking_field ? 0.0f : p.sticking, qs = q.s.sticking_field ? 0.0f : q.sticking;
+    if (ps != qs) return ps < qs;
+    return depth(p) > depth(q);
+  });
+  return order;
+}
+
 int build_tables(rtg_batch* b) {
   rtg_context* ctx = &b->aux;
   const int n = (int)b->jobs.size();
   std::vector<TraceParams> h(n);
   std::vector<uint64_t> prefix(n + 1, 0);
-  for (int j = 0; j < n; ++j) {
-    h[j] = b->jobs[j].p;
-    prefix[j + 1] = prefix[j] + b->jobs[j].n_rays;
+  const std::vector<int> order = launch_order(b);
+  for (int i = 0; i < n; ++i) {
+    const Job& j = b->jobs[order[i]];
+    h[i] = j.p;
+    prefix[i + 1] = prefix[i] + j.n_rays;
   }
   b->total_rays = prefix[n];
   RTG_TRY(dalloc(ctx, b->d_jobs, (size_t)(n > 0 ? n : 1), "batch job table"));
@@ -96,7 +118,21 @@ int enqueue_batched(rtg_batch* b, cudaStream_t st, const uint64_t* prefix, uint6
   if (total > 0)
     RTG_TRY(launch_trace_batched(ctx, p0, b->d_jobs.p, prefix, (int)b->jobs.size(), total, st, ctx->lc, b->depth,
                                  b->wide));
-  for (Job& j : b->jobs) RTG_TRY(compute_areas_into(j.scene, st, j.box_lo, j.box_hi, j.areas.p));
+  // one pass a surface and box: the species of a surface share them (20 us a pass)
+  for (size_t i = 0; i < b->jobs.size(); ++i) {
+    Job& j = b->jobs[i];
+    const Job* same = nullptr;
+    for (size_t k = i; k > 0 && i - k < 64 && !same;) {  // no further back: the search stays linear
+      const Job& o = b->jobs[--k];
+      if (o.scene == j.scene && std::equal(o.box_lo, o.box_lo + 3, j.box_lo) &&
+          std::equal(o.box_hi, o.box_hi + 3, j.box_hi))
+        same = &o;
+    }
+    if (same)
+      RTG_CUDA(ctx, cudaMemcpyAsync(j.areas.p, same->areas.p, j.np * sizeof(float), cudaMemcpyDeviceToDevice, st));
+    else
+      RTG_TRY(compute_areas_into(j.scene, st, j.box_lo, j.box_hi, j.areas.p));
+  }
   return RTG_OK;
 }
 
@@ -412,11 +448,12 @@ static int rtg_batch_autotune_body(rtg_batch* b, double fraction, rtg_launch_con
   if (n == 0) return set_error(ctx, RTG_ERR_INVALID_ARGUMENT, "empty batch");
   // the first fraction of every job's rays
   std::vector<uint64_t> prefix(n + 1, 0);
-  for (int j = 0; j < n; ++j) {
-    const uint64_t r = b->jobs[j].n_rays;
+  const std::vector<int> jobs = launch_order(b);
+  for (int i = 0; i < n; ++i) {
+    const uint64_t r = b->jobs[jobs[i]].n_rays;
     uint64_t s = (uint64_t)(r * fraction);
     if (s == 0 && r > 0) s = 1;
-    prefix[j + 1] = prefix[j] + s;
+    prefix[i + 1] = prefix[i] + s;
   }
   const uint64_t total = prefix[n];
   DBuf<uint64_t> dp;
