@@ -59,7 +59,7 @@ def workload():
 
 
 TREE = "ploc"  # --tree: PLOC clustering traces the hole 4 % faster than the radix tree and builds in 1.8 ms
-NODE_WIDTH = 0   # --node-width: 0 automatic (binary for this L2-resident hole), 2 binary, 8 wide
+NODE_WIDTH = 0   # --node-width: 0 automatic (as 2), 2 four-box nodes of the binary tree, 8 wide
 
 
 def set_tree(name, node_width=0):
@@ -84,6 +84,12 @@ def read_peaks():
         return float(d["hbm_gbs"]), "measured"
     except Exception:
         return 6800.0, "fallback"
+
+
+def launches_per_step(rays):
+    """Kernels of one trace of the hole: path kernel and areas, and from 2^21 rays the
+    three that order the rays (count, scan, place)."""
+    return 5 if rays >= 1 << 21 else 2
 
 
 def read_profile_line(key):
@@ -610,7 +616,7 @@ def run_ours(args):
                 "scaling": "weak", "vs_baseline": None, "dtype": "f32 paths, f64 accumulators",
                 "data": "synthetic", "config": config_dict(h, R), "clocks": clocks, "roofline": roof,
                 "roofline_l2": roof_l2,
-                "cpu_baseline": cpu, "e2e": e2e, "gpu_launches": 2 * args.steps, "adjoint": adj,
+                "cpu_baseline": cpu, "e2e": e2e, "gpu_launches": launches_per_step(R) * args.steps, "adjoint": adj,
                 "plain_gpu": plain, "batch": batch, "rough_field": rough, "flux_error": flux_err,
                 "flux_1pct": one_pct,
                 "wall_s_timed_region": wall,

@@ -100,8 +100,7 @@ struct SceneView {
   const float4* tri;
   int32_t nt;
   const float4* basis;  // by slot, discs then triangles, 32 B each: the basis of the normal (pack_basis)
-  const Node* nodes;       // the binary tree (the window deposit's interval queries)
-  const QuadNode* quads;   // the same tree as closest hits visit it, up to four boxes a node
+  const QuadNode* quads;   // the tree as queries visit it, up to four boxes a node
   uint32_t root;        // child reference of the root (internal node 0 or a leaf)
   // the 8-wide compressed tree of the closest-hit query (root = wide node 0),
   // or nullptr: closest hits visit the quads

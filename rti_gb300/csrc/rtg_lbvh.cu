@@ -7,14 +7,16 @@
 //   3. stable radix sort (rtg_sort.cu),
 //   4. Karras (HPG 2012) binary radix tree over the keys (morton << 32 | rank),
 //   5. primitives copied to slot order (LBVH leaf order) for coherent access,
-//   6. bottom-up box refit with per-node arrival counters.
-// rtg_update_* reruns 1, 5 and 6 only (moved surface, same topology).
-// Step 4 is by default replaced by PLOC clustering over the same sorted
-// leaves (build_ploc), whose trees need fewer node visits per query.
+//   6. bottom-up box refit with per-node arrival counters,
+//   7. the four-box node of every internal node, and the stack these can need.
+// rtg_update_* reruns 1, 5, 6 and 7 only (moved surface, same topology).
+// Step 4 can be replaced by PLOC clustering over the same sorted leaves
+// (build_ploc), whose trees need fewer node visits per query on irregular
+// surfaces and take longer to build.
 //
 // Leaves hold one primitive; each internal node stores the boxes of both
-// children (64 bytes).  Closest hits visit QuadNodes instead, which the refit
-// makes on its way up: up to four boxes below the node in one fetch.
+// children (64 bytes), from which step 7 takes up to four boxes below the node
+// in one fetch (QuadNode).
 #include <cfloat>
 #include <cstdint>
 #include <vector>

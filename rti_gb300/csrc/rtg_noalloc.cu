@@ -1,12 +1,11 @@
 // rtg_noalloc.cu -- normalised, smoothed estimates without any device allocation.
 //
-// rtg_get_mc_estimates allocates a small device scratch buffer for the
-// maximum on every call and frees it again; cudaFree synchronises the whole
-// device.  Some callers cannot allocate device memory at that point: a
+// rtg_get_mc_estimates keeps a buffer for the maximum and the flux in the
+// context, which its first call on a surface allocates, and waits for the
+// result.  Some callers cannot allocate device memory at that point: a
 // process simulator that keeps every byte of the GPU under its own memory
 // pool (and must not grow it behind the pool's back), or one that overlaps
-// the next surface update with the flux finalisation and cannot afford the
-// device-wide synchronisation of cudaFree.  rtg_get_mc_estimates_noalloc
+// the next surface update with the flux finalisation and must not wait.  rtg_get_mc_estimates_noalloc
 // computes the same estimates (device.hpp:154-187) into a device buffer the
 // caller owns, and keeps its scratch -- one maximum per 256-element block
 // plus the overall maximum -- in the file-scope array below.

@@ -309,7 +309,8 @@ __device__ __forceinline__ bool closest_hit_wide(const SceneView& s, const Ray& 
 // nodes (two boxes and two loads a visit, lo/hi planes), over 128-byte quads
 // (four loads), over these (three): trench 1e6 rays 3.13, 2.23, 2.19 ms; hole
 // (200 k triangles) 1e6 rays 17.7, 13.8, 13.8 and 1e7 rays 52.2, 46.9, 44.1; 2e7
-// rays onto 4.19 M discs 30.5 (8-wide tree), 27.6, 25.8.  64-byte quads (two
+// rays onto 4.19 M discs 30.5 (8-wide tree), 27.6, 25.8; with everything else
+// as it is now 1.91, 13.1, 39.9 and 15.9.  64-byte quads (two
 // loads, 16-bit centres in a frame of the surface) cost 12 to 24 byte permutes a
 // visit and wider boxes: 2.35, 14.4, 46.6, 25.5.
 // Boxes that the ray leaves before tnear are skipped, since a hit
@@ -628,9 +629,9 @@ __device__ __forceinline__ double warp_sum_d(double v) {
 }
 
 // Threads per SM that the register target leaves room for.  Forward: 1024 (64
-// registers, nothing spilled); 1152 and 896 measured 2.36 and 2.22 against
-// 2.20 ms on the 98 k-disc trench (1e6 rays), 27.1 and 29.7 against 26.5 ms on
-// 4.19 M discs.  The global adjoint: 768 (80 registers; at 64 it spills 138 B):
+// registers, nothing spilled); 1152 and 896 measured 2.25 and 2.19 against
+// 2.13 ms on the 98 k-disc trench (1e6 rays), 44.5 and 43.9 against 43.5 into the
+// hole (1e7), 24.8 and 28.3 against 25.8 onto 4.19 M discs (2e7).  The global adjoint: 768 (80 registers; at 64 it spills 138 B):
 // 1e6 rays into the hole 14.8 -> 13.8 ms, trench 2.66 -> 2.51; the field adjoint
 // loses more by the missing warps (4.19 M discs 7.96 -> 9.12 ms) and keeps 1024.
 // The window mode: 768 (nothing spilled; at 64 registers 76 B): 300 007 rays into a

@@ -11,9 +11,8 @@ namespace {
 constexpr int kQueryThreads = 128;
 
 // Closest hits of explicit rays, `share` of them a warp, bound as a trace's
-// queries are.  The stack follows the tree's need (a 256-entry one in every
-// thread and the wide traversal compiled in went with 230 us more a call).
-// Whole calls of 262 144 rays, before -> now: hole of 31 k triangles 479 -> 219 us,
+// queries are.  The stack follows the tree's need, and the wide traversal is
+// compiled in only where it runs.  Whole calls of 262 144 rays, before -> now: hole of 31 k triangles 479 -> 219 us,
 // trench of 98 k discs 488 -> 198, 4.19 M discs 707 -> 379; 1000 rays 106 -> 81.
 // 768, 1280 and 1536 threads an SM: 230, 224, 245 us for the hole.
 template <int STACK, bool WIDE>
@@ -218,7 +217,6 @@ SceneView scene_view(rtg_context* ctx) {
   s.nd = (int32_t)g.nd;
   s.tri = g.tri.p;
   s.nt = (int32_t)g.nt;
-  s.nodes = g.nodes.p;
   s.quads = g.quads.p;
   s.basis = g.basis.p;
   s.root = g.root;
