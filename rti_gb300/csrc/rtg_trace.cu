@@ -304,7 +304,10 @@ int launch_trace(rtg_context* ctx, const TraceParams& p_in, cudaStream_t st, int
   // one launch, or several of ordered rays
   uint64_t chunk = nrays;
   DBuf<uint32_t>& ids = ctx->ray_order[mode == kModeAdjGlobal || mode == kModeAdjField ? 1 : 0];
-  bool ordered = mode != kModeLogged && wants_order(ctx, p, nrays);
+  // the context's own traces and replays only: a batch's launches with its scenes' contexts may be on several
+  // streams at once, and would share the ids
+  const bool own = p.tally == ctx->d_tally || p.tally == ctx->d_tally_adj;
+  bool ordered = own && mode != kModeLogged && wants_order(ctx, p, nrays);
   if (ordered) {
     const uint64_t chunks = (nrays + kOrderMax - 1) / kOrderMax;
     chunk = (nrays + chunks - 1) / chunks;

@@ -115,6 +115,30 @@ def test_adjoint_equals_pieces(eng, field):
     np.testing.assert_allclose(out[0][1], out[1][1], rtol=1e-9, atol=1e-9 * n)
 
 
+def test_batches_of_one_scene_on_two_streams(rtg_lib):
+    """Sequential launches of two batches that share a context, on two streams at
+    once: they keep no ray order in it, so neither disturbs the other."""
+    import torch
+    from rti_gb300 import Engine
+    from rti_gb300.batch import Batch
+    e, bs = Engine(0), [Batch(0), Batch(0)]
+    try:
+        _deep(e)
+        rays = [(1 << 21) + 7, (1 << 21) + 4099]
+        jobs = [b.add(e, r, seed=3 + i, config=e.config()) for i, (b, r) in enumerate(zip(bs, rays))]
+        streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+        for b, s in zip(bs, streams):
+            b.run_sequential(stream=s.cuda_stream)
+        torch.cuda.synchronize()
+        for i, (b, j, r) in enumerate(zip(bs, jobs, rays)):
+            e.trace(r, 3 + i)
+            assert np.array_equal(b.results(j)[1], e.hit_counts())
+    finally:
+        for b in bs:
+            b.close()
+        e.close()
+
+
 def test_without_room_the_rays_are_taken_in_ascending_order(rtg_lib):
     from rti_gb300 import Engine
     with Engine(0) as e:
