@@ -315,10 +315,10 @@ int launch_trace(rtg_context* ctx, const TraceParams& p_in, cudaStream_t st, int
     if (!ordered) chunk = nrays;
   }
   const uint64_t end = p.ray_end;
-  for (uint64_t begin = p.ray_begin; begin < end; begin += chunk) {
+  for (uint64_t begin = p.ray_begin; begin < end;) {
+    const uint64_t n = std::min(chunk, end - begin);  // begin + chunk may pass 2^64
     p.ray_begin = begin;
-    p.ray_end = std::min(end, begin + chunk);
-    const uint64_t n = p.ray_end - p.ray_begin;
+    p.ray_end = begin + n;
     if (ordered) {
       const unsigned grid = (unsigned)((n + 255) / 256);
       uint32_t* cells = ids.p;
@@ -336,7 +336,7 @@ int launch_trace(rtg_context* ctx, const TraceParams& p_in, cudaStream_t st, int
     if (blocks > 0x7FFFFFFFull) return set_error(ctx, RTG_ERR_INVALID_ARGUMENT, "too many rays for a plain launch");
     kern<<<(unsigned)blocks, tpb, 0, st>>>(p, nullptr, nullptr, 0);
     RTG_CUDA(ctx, cudaGetLastError());
-    if (end - begin <= chunk) break;  // begin + chunk may pass 2^64
+    begin += n;
   }
   return RTG_OK;
 }
