@@ -315,6 +315,8 @@ __device__ __forceinline__ bool closest_hit_wide(const SceneView& s, const Ray& 
 // visit and wider boxes: 2.35, 14.4, 46.6, 25.5.
 // Boxes that the ray leaves before tnear are skipped, since a hit
 // needs t > tnear: a ray that starts on a flat face passes over the whole face.
+// With a negative tnear (explicit rays) boxes behind the origin are skipped, as in
+// the wide tree.
 // Leaf children hit are tested on the spot; of the inner ones the nearest is
 // visited next and the others wait on the stack, nearly sorted (near child of
 // each pair, then the near pair).
@@ -343,7 +345,7 @@ __device__ bool closest_hit(const SceneView& s, f3 o, f3 d, float tnear, float& 
   uint32_t cur = s.root;
   const uint32_t max_iter = s.max_visits;
   const QuadRay qr = quad_ray(r);
-  const float tmin = tnear * 0.999999f;
+  const float tmin = fmaxf(tnear, 0.0f) * 0.999999f;
   for (uint32_t it = 0;; ++it) {
     if (it >= max_iter || (kChecked && !node_in_range(s, cur))) {
       errs += 1;
