@@ -336,16 +336,16 @@ static void build_rec(orc_scene* s, int64_t ni, int64_t first, int64_t count) {
   build_rec(s, r, mid, first + count - mid);
 }
 
-/* Conservative primitive boxes: exact extents padded so that any hit the
- * primitive test accepts lies inside the box. */
+/* Conservative primitive boxes: extents padded so that any hit the primitive
+ * test accepts lies inside the box.  A disc reaches r sqrt(n_j^2 + n_k^2) / |n|
+ * along axis i, and its normal may be off unit length by 1e-3. */
 static void prim_boxes(orc_scene* s) {
   for (int64_t i = 0; i < s->nd; ++i) {
     float r = s->dc[4 * i + 3];
     for (int a = 0; a < 3; ++a) {
-      float n = s->dn[3 * i + a];
+      float n = s->dn[3 * i + a], nj = s->dn[3 * i + (a + 1) % 3], nk = s->dn[3 * i + (a + 2) % 3];
       float c = s->dc[4 * i + a];
-      float e = 1.0f - n * n;
-      float ext = r * sqrtf(e > 0.0f ? e : 0.0f);
+      float ext = r * sqrtf(fmaxf(1.0f - n * n, nj * nj + nk * nk));
       float pad = 1e-5f * (fabsf(c) + r) + 1e-4f * r;
       s->blo[3 * i + a] = c - ext - pad;
       s->bhi[3 * i + a] = c + ext + pad;

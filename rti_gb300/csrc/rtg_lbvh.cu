@@ -36,8 +36,11 @@ __device__ __forceinline__ float fdec(uint32_t u) {
   return __uint_as_float((u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u);
 }
 
-// Conservative boxes: the exact extent of the disc (r*sqrt(1-n_i^2)) or of the
-// triangle, padded so that every hit the primitive test accepts lies inside.
+// Conservative boxes: the extent of the disc or of the triangle, padded so that
+// every hit the primitive test accepts lies inside.  A disc reaches r
+// sqrt(n_j^2 + n_k^2) / |n| along axis i; its normal may be off unit length by
+// 1e-3, and max(1 - n_i^2, n_j^2 + n_k^2) is never below that square (1 - n_i^2
+// is where |n| <= 1, the other where |n| >= 1).
 constexpr int kBoundsThreads = 256;
 __global__ void __launch_bounds__(kBoundsThreads) prim_bounds_kernel(const float4* __restrict__ dcr, const float4* __restrict__ dn, int64_t nd,
                                    const float4* __restrict__ tv, const uint32_t* __restrict__ tidx,
@@ -52,8 +55,9 @@ __global__ void __launch_bounds__(kBoundsThreads) prim_bounds_kernel(const float
       float cc[3] = {c.x, c.y, c.z}, nn[3] = {n.x, n.y, n.z};
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
-        float e = 1.0f - nn[a] * nn[a];
-        float ext = c.w * sqrtf(e > 0.0f ? e : 0.0f);
+        const float nj = nn[(a + 1) % 3], nk = nn[(a + 2) % 3];
+        const float e = fmaxf(1.0f - nn[a] * nn[a], nj * nj + nk * nk);
+        float ext = c.w * sqrtf(e);
         float pad = 1e-5f * (fabsf(cc[a]) + c.w) + 1e-4f * c.w;
         lo[a] = cc[a] - ext - pad;
         hi[a] = cc[a] + ext + pad;
