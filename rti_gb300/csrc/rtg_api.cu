@@ -510,22 +510,23 @@ size_t build_scratch(const rtg_context* ctx, int64_t nd, int64_t nv, int64_t nt)
   return (size_t)(160 * nd + 28 * nv + 12 * nt + 96 * np + (ctx->g.builder == kBuilderPloc ? 96 * np : 0)) + 262144;
 }
 
-// The tree (built anew, or refitted in place) and the neighbour lists; waits
-// until they are complete.
-int rebuild(rtg_context* ctx, bool refit) {
+// The tree (built anew, or refitted in place) and the neighbour lists (unless
+// discs and slots are as they were: a refit for moved vertices); waits until they
+// are complete.
+int rebuild(rtg_context* ctx, bool refit, bool neighbors) {
   NeighborWork w;
-  int rc = count_neighbors(ctx, w);
+  int rc = neighbors ? count_neighbors(ctx, w) : RTG_OK;
   if (rc == RTG_OK) rc = refit ? refit_lbvh(ctx) : build_lbvh(ctx);
-  if (rc == RTG_OK) rc = fill_neighbors(ctx, w);
+  if (rc == RTG_OK && neighbors) rc = fill_neighbors(ctx, w);
   release_neighbors(w, ctx->stream);
   const cudaError_t e = cudaStreamSynchronize(ctx->stream);
   if (rc == RTG_OK && e != cudaSuccess) rc = check_cuda(ctx, e, "surface build");
   return rc;
 }
 
-int rebuild_all(rtg_context* ctx, bool refit) {
+int rebuild_all(rtg_context* ctx, bool refit, bool neighbors = true) {
   RTG_TRY(alloc_results(ctx));
-  RTG_TRY(rebuild(ctx, refit));
+  RTG_TRY(rebuild(ctx, refit, neighbors));
   resolve_box(ctx);
   return RTG_OK;
 }
@@ -719,7 +720,7 @@ static int rtg_update_vertices_body(rtg_context* ctx, const float* vertices, int
   rc = check_cuda(ctx, cudaMemcpyAsync(g.tri_v.p, sg.v4.p, nv * sizeof(float4), cudaMemcpyDeviceToDevice, ctx->stream),
                   "vertex update");
   release(sg, ctx->stream);
-  if (rc == RTG_OK) rc = rebuild_all(ctx, true);
+  if (rc == RTG_OK) rc = rebuild_all(ctx, true, false);
   if (rc != RTG_OK) drop_surface(ctx);
   return rc;
 }
@@ -841,7 +842,7 @@ int rtg_set_tree_builder(rtg_context* ctx, int32_t builder) {
   if (ctx->g.nd + ctx->g.nt > 0 && ctx->g.nodes.p && builder != keep) {
     ++ctx->version;
     int rc = check_cuda(ctx, cudaStreamSynchronize(ctx->stream), "tree rebuild");
-    if (rc == RTG_OK) rc = rebuild(ctx, false);  // neighbour columns are stored as slots of the new tree
+    if (rc == RTG_OK) rc = rebuild(ctx, false, true);  // neighbour columns are stored as slots of the new tree
     if (rc != RTG_OK) {
       drop_surface(ctx);
       return rc;
