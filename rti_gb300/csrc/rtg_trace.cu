@@ -27,7 +27,8 @@ __global__ void __launch_bounds__(kQueryThreads, 1024 / kQueryThreads)
   int id;
   uint32_t ref;
   uint32_t e = 0;
-  if (closest_hit<STACK, 0, WIDE>(s, mk3(r[0], r[1], r[2]), mk3(r[3], r[4], r[5]), tnear, t, id, ref, e)) {
+  if (closest_hit<STACK, 0, WIDE>(s, mk3(r[0], r[1], r[2]), mk3(r[3], r[4], r[5]), tnear, fmaxf(tnear, 0.0f), t, id,
+                                  ref, e)) {
     prim[i] = id;
     tout[i] = t;
   } else {
