@@ -422,8 +422,17 @@ int commit(rtg_context* ctx, const Staged& sg) {
 
 }  // namespace
 
+void release_kept(rtg_context* ctx) {
+  cudaDeviceSynchronize();  // what a launch in flight has taken comes back with its end
+  if (ctx->order_pool) cudaMemPoolTrimTo(ctx->order_pool, 0);
+  dfree(ctx->queries);
+  if (!ctx->scratch_open) dfree(ctx->scratch);
+  cudaGetLastError();
+}
+
 void drop_surface(rtg_context* ctx) {
   cudaStreamSynchronize(ctx->stream);
+  release_kept(ctx);
   Geometry& g = ctx->g;
   dfree(g.disc_cr_by_id); dfree(g.disc_n_by_id); dfree(g.tri_v); dfree(g.tri_idx);
   dfree(g.disc); dfree(g.tri); dfree(g.basis); dfree(g.nodes); dfree(g.quads);
@@ -629,7 +638,7 @@ int rtg_destroy(rtg_context* ctx) {
   dfree(ctx->stat_tmp);
   dfree(ctx->scratch);
   dfree(ctx->queries);
-  for (auto& b : ctx->ray_order) dfree(b);
+  if (ctx->order_pool) cudaMemPoolDestroy(ctx->order_pool);
   dfree(g.wnodes);
   dfree(ctx->seglog);
   dfree(ctx->seglog_count);
@@ -1288,6 +1297,7 @@ int rtg_trace_rays(rtg_context* ctx, const float* rays, int64_t n, float tnear, 
   DBuf<unsigned char>& q = ctx->queries;
   const size_t rays_at = 0, t_at = 24 * (size_t)n, prim_at = 28 * (size_t)n, err_at = (32 * (size_t)n + 7) / 8 * 8;
   if (n > (int64_t)1 << 48) return set_error(ctx, RTG_ERR_OUT_OF_MEMORY, "no room for the ray queries");
+  RTG_TRY(ensure_wide(ctx));  // before the buffer: an allocation that fails gives the buffer back
   if (q.n < err_at + 8) RTG_TRY(dalloc(ctx, q, (err_at + 8 + 65535) / 65536 * 65536, "ray queries"));
   float* d_rays = reinterpret_cast<float*>(q.p + rays_at);
   float* d_t = reinterpret_cast<float*>(q.p + t_at);

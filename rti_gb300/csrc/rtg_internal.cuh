@@ -251,7 +251,7 @@ struct rtg_context {
   rtg::DBuf<unsigned char> scratch;
   size_t scratch_top = 0;
   bool scratch_open = false;
-  rtg::DBuf<uint32_t> ray_order[2];  // cells | ray ids of an ordered launch (trace, adjoint), kept; see launch_trace
+  cudaMemPool_t order_pool = nullptr;  // cells | ray ids of ordered launches; see launch_trace
   rtg::DBuf<unsigned char> queries;  // rtg_trace_rays: rays and results of a call, at most kScratchMax kept
   // segment log (rtg_set_segment_log)
   rtg::DBuf<rtg_segment> seglog;
@@ -392,6 +392,10 @@ int host_guard(rtg_context* ctx, F&& f) noexcept {
     }
   }
 }
+// Gives back the device memory that the context keeps for speed alone and that no
+// call uses now: the room of ordered launches, the buffer of explicit rays, the
+// scratch of builds.
+void release_kept(rtg_context* ctx);
 // Fault injection (rtg_inject_alloc_failure): whether this allocation is the
 // one chosen to fail.
 inline bool injected_alloc_failure(rtg_context* ctx) {
@@ -408,9 +412,16 @@ int dalloc(rtg_context* ctx, DBuf<T>& b, size_t n, const char* what) {
   b.p = nullptr;
   b.n = 0;
   if (n == 0) return RTG_OK;
-  if (injected_alloc_failure(ctx))
+  if (injected_alloc_failure(ctx)) {
+    release_kept(ctx);
     return set_error(ctx, RTG_ERR_OUT_OF_MEMORY, std::string("cudaMalloc failed for ") + what + " (injected)");
+  }
   cudaError_t e = cudaMalloc((void**)&b.p, n * sizeof(T));
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    release_kept(ctx);
+    e = cudaMalloc((void**)&b.p, n * sizeof(T));
+  }
   if (e != cudaSuccess) {
     b.p = nullptr;
     cudaGetLastError();
@@ -478,6 +489,11 @@ int talloc(rtg_context* ctx, DBuf<T>& b, size_t n, cudaStream_t st, const char* 
     }
   }
   cudaError_t e = cudaMallocAsync((void**)&b.p, n * sizeof(T), st);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    release_kept(ctx);
+    e = cudaMallocAsync((void**)&b.p, n * sizeof(T), st);
+  }
   if (e != cudaSuccess) {
     b.p = nullptr;
     cudaGetLastError();

@@ -43,7 +43,8 @@ __global__ void __launch_bounds__(kQueryThreads, 1024 / kQueryThreads)
 // nodes.  A cell is one of 64 x 64 parts of the source rectangle (in Morton order)
 // and a quarter turn of the direction, all of them high bits of the source draw.
 constexpr int kCellBits = 6, kTurnBits = 2, kCells = 1 << (2 * kCellBits + kTurnBits);
-constexpr uint64_t kOrderMax = 1u << 25;  // rays ordered at once (128 MB of ids)
+constexpr uint64_t kOrderMax = 1u << 25;     // rays ordered at once (128 MB of ids)
+constexpr uint64_t kOrderKept = 128u << 20;  // bytes that a context keeps for its next ordered launch
 
 __device__ __forceinline__ uint32_t spread_bits(uint32_t v) {  // 6 bits to every second place
   v = (v | v << 4) & 0x0F0Fu;
@@ -250,26 +251,68 @@ bool wants_order(const rtg_context* ctx, const TraceParams& p, uint64_t nrays) {
   return nrays >= 1u << 21 && p.box_hi[2] - p.box_lo[2] >= wide;
 }
 
-// Room for the cells and the ids of an ordered launch, kept by the context (at
-// most 128 MB).  Without it, or while the stream is being captured (the buffer may
-// be another one when the graph runs), the launch takes its rays in ascending order.
-bool room_for_order(rtg_context* ctx, DBuf<uint32_t>& ids, cudaStream_t st, uint64_t rays) {
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+// A capture of another stream has no part in the pool, so it may go on meanwhile:
+// the calls are made with this thread's capture mode relaxed.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  RelaxedCapture(const RelaxedCapture&) = delete;
+  RelaxedCapture& operator=(const RelaxedCapture&) = delete;
+};
+
+// The cells and the ids of an ordered launch, taken from the context's pool and
+// given back to it in the order of the stream, so that the call only enqueues: a
+// buffer of cudaMalloc made a larger launch than before wait for the one before it,
+// and broke a capture that another stream had open in the global mode.  The pool
+// keeps kOrderKept bytes between launches (mapping 80 MB anew takes 0.3 ms of the
+// 16 ms of 2e7 rays onto 4.19 M discs, 12 MB 0.18 ms of the 2 of 3e6) and gives
+// them up in release_kept.
+struct OrderRoom {
+  uint32_t* p = nullptr;
+  cudaStream_t st;
+  explicit OrderRoom(cudaStream_t s) : st(s) {}
+  ~OrderRoom() {
+    if (!p) return;
+    const RelaxedCapture relaxed;
+    cudaFreeAsync(p, st);
+  }
+  OrderRoom(const OrderRoom&) = delete;
+  OrderRoom& operator=(const OrderRoom&) = delete;
+
+  // Whether there is room.  Without it, or while the stream is being captured (a
+  // graph would hold the room for as long as it lives), the launch takes its rays in
+  // ascending order.
+  bool take(rtg_context* ctx, uint64_t rays) {
+    const RelaxedCapture relaxed;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone &&
+        !injected_alloc_failure(ctx) && make_pool(ctx) &&
+        cudaMallocFromPoolAsync((void**)&p, (kCells + (size_t)rays) * sizeof(uint32_t), ctx->order_pool, st) == cudaSuccess)
+      return true;
     cudaGetLastError();
+    p = nullptr;
     return false;
   }
-  const size_t words = kCells + (size_t)rays;
-  if (ids.n >= words) return true;
-  dfree(ids);
-  if (injected_alloc_failure(ctx) || cudaMalloc((void**)&ids.p, words * sizeof(uint32_t)) != cudaSuccess) {
-    cudaGetLastError();
-    ids.p = nullptr;
-    return false;
+
+ private:
+  static bool make_pool(rtg_context* ctx) {
+    if (ctx->order_pool) return true;
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = ctx->device;
+    if (cudaMemPoolCreate(&ctx->order_pool, &props) != cudaSuccess) {
+      ctx->order_pool = nullptr;
+      return false;
+    }
+    uint64_t keep = kOrderKept;
+    int off = 0;  // a trace and a replay on two streams do not wait for each other's room
+    cudaMemPoolSetAttribute(ctx->order_pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    cudaMemPoolSetAttribute(ctx->order_pool, cudaMemPoolReuseAllowInternalDependencies, &off);
+    return true;
   }
-  ids.n = words;
-  return true;
-}
+};
 
 }  // namespace
 
@@ -304,15 +347,15 @@ int launch_trace(rtg_context* ctx, const TraceParams& p_in, cudaStream_t st, int
   if (per_sm < 1) per_sm = 1;
   // one launch, or several of ordered rays
   uint64_t chunk = nrays;
-  DBuf<uint32_t>& ids = ctx->ray_order[mode == kModeAdjGlobal || mode == kModeAdjField ? 1 : 0];
-  // the context's own traces and replays only: a batch's launches with its scenes' contexts may be on several
-  // streams at once, and would share the ids
+  OrderRoom room(st);
+  // the context's own traces and replays only: two batches that share a scene's context may launch from two threads,
+  // and must not both make its pool
   const bool own = p.tally == ctx->d_tally || p.tally == ctx->d_tally_adj;
   bool ordered = own && mode != kModeLogged && wants_order(ctx, p, nrays);
   if (ordered) {
     const uint64_t chunks = (nrays + kOrderMax - 1) / kOrderMax;
     chunk = (nrays + chunks - 1) / chunks;
-    ordered = room_for_order(ctx, ids, st, chunk);
+    ordered = room.take(ctx, chunk);
     if (!ordered) chunk = nrays;
   }
   const uint64_t end = p.ray_end;
@@ -322,12 +365,12 @@ int launch_trace(rtg_context* ctx, const TraceParams& p_in, cudaStream_t st, int
     p.ray_end = begin + n;
     if (ordered) {
       const unsigned grid = (unsigned)((n + 255) / 256);
-      uint32_t* cells = ids.p;
-      p.order = ids.p + kCells;
+      uint32_t* cells = room.p;
+      p.order = room.p + kCells;
       RTG_CUDA(ctx, cudaMemsetAsync(cells, 0, kCells * sizeof(uint32_t), st));
       order_count_kernel<<<grid, 256, 0, st>>>(p, (uint32_t)n, cells);
       RTG_TRY(exclusive_scan_u32(ctx, cells, kCells, nullptr, st));
-      order_place_kernel<<<grid, 256, 0, st>>>(p, (uint32_t)n, cells, ids.p + kCells);
+      order_place_kernel<<<grid, 256, 0, st>>>(p, (uint32_t)n, cells, room.p + kCells);
     }
     if (begin != p_in.ray_begin)
       RTG_CUDA(ctx, cudaMemsetAsync(&p.tally->next_ray, 0, sizeof(unsigned long long), st));
@@ -345,7 +388,6 @@ int launch_trace(rtg_context* ctx, const TraceParams& p_in, cudaStream_t st, int
 int launch_closest_hit(rtg_context* ctx, const float* d_rays, int64_t n, float tnear, int32_t* d_prim, float* d_t,
                        unsigned long long* d_errors, cudaStream_t st) {
   if (n <= 0) return RTG_OK;
-  RTG_TRY(ensure_wide(ctx));
   const SceneView s = scene_view(ctx);
   const int stack = stack_for(0, traversal_depth(ctx));
   int sms = 0;
