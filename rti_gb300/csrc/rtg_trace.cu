@@ -42,8 +42,16 @@ __global__ void __launch_bounds__(kQueryThreads, 1024 / kQueryThreads)
 // so that a warp's paths, and those in flight around them, visit the same
 // nodes.  A cell is one of 64 x 64 parts of the source rectangle (in Morton order)
 // and a quarter turn of the direction, all of them high bits of the source draw.
+// The rays are sorted in pieces, one after the other in the order that the launch
+// takes them: of more rays a cell holds so many that all paths in flight deposit on
+// the same few primitives.  4e8 rays, sorted as one piece -> in pieces of 2^25, one
+// launch -> a launch for each piece, which lets the GPU run empty after each:
+// directional source on a disc hole 295 -> 221 -> 219 ms, hole of 200 k triangles
+// 1256 -> 1280 -> 1362, trench 437 -> 439 -> 442, 4.19 M discs 313 -> 317 -> 317 (in
+// ascending order 279, 1295, 444, 413).
 constexpr int kCellBits = 6, kTurnBits = 2, kCells = 1 << (2 * kCellBits + kTurnBits);
-constexpr uint64_t kOrderMax = 1u << 25;     // rays ordered at once (128 MB of ids)
+constexpr uint64_t kOrderPiece = 1u << 25;   // rays sorted at once
+constexpr uint64_t kOrderMax = 1u << 29;     // rays of one launch (2 GB of ids)
 constexpr uint64_t kOrderKept = 128u << 20;  // bytes that a context keeps for its next ordered launch
 
 __device__ __forceinline__ uint32_t spread_bits(uint32_t v) {  // 6 bits to every second place
@@ -56,16 +64,18 @@ __device__ __forceinline__ uint32_t source_cell(const TraceParams& p, uint32_t j
   const uint32_t place = spread_bits(u.x >> (32 - kCellBits)) << 1 | spread_bits(u.y >> (32 - kCellBits));
   return place << kTurnBits | u.z >> (32 - kTurnBits);
 }
-// One thread per ray, bound by the atomics on the cells (2e7 rays: 0.12 ms to
-// count, 0.23 ms to place; the trace of these takes 13 to 16 ms).
-__global__ void order_count_kernel(const __grid_constant__ TraceParams p, uint32_t n, uint32_t* __restrict__ cells) {
+// One thread per ray of the piece that begins with the launch's ray `first`, bound
+// by the atomics on the cells (2e7 rays: 0.12 ms to count, 0.23 ms to place; the
+// trace of these takes 13 to 16 ms).
+__global__ void order_count_kernel(const __grid_constant__ TraceParams p, uint32_t first, uint32_t n,
+                                   uint32_t* __restrict__ cells) {
   const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j < n) atomicAdd(&cells[source_cell(p, j)], 1u);
+  if (j < n) atomicAdd(&cells[source_cell(p, first + j)], 1u);
 }
-__global__ void order_place_kernel(const __grid_constant__ TraceParams p, uint32_t n, uint32_t* __restrict__ cells,
-                                   uint32_t* __restrict__ order) {
+__global__ void order_place_kernel(const __grid_constant__ TraceParams p, uint32_t first, uint32_t n,
+                                   uint32_t* __restrict__ cells, uint32_t* __restrict__ order) {
   const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j < n) order[atomicAdd(&cells[source_cell(p, j)], 1u)] = j;
+  if (j < n) order[first + atomicAdd(&cells[source_cell(p, first + j)], 1u)] = first + j;
 }
 
 template <int TPB>
@@ -251,6 +261,12 @@ bool wants_order(const rtg_context* ctx, const TraceParams& p, uint64_t nrays) {
   return nrays >= 1u << 21 && p.box_hi[2] - p.box_lo[2] >= wide;
 }
 
+// The size of equal parts of n, as few as keep each within most.
+uint64_t equal_parts(uint64_t n, uint64_t most) {
+  const uint64_t parts = n / most + (n % most != 0);
+  return n / parts + (n % parts != 0);
+}
+
 // A capture of another stream has no part in the pool, so it may go on meanwhile:
 // the calls are made with this thread's capture mode relaxed.
 struct RelaxedCapture {
@@ -345,7 +361,7 @@ int launch_trace(rtg_context* ctx, const TraceParams& p_in, cudaStream_t st, int
   RTG_CUDA(ctx, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
   RTG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, tpb, 0));
   if (per_sm < 1) per_sm = 1;
-  // one launch, or several of ordered rays
+  // one launch, or several of more ordered rays than a launch may have
   uint64_t chunk = nrays;
   OrderRoom room(st);
   // the context's own traces and replays only: two batches that share a scene's context may launch from two threads,
@@ -353,8 +369,7 @@ int launch_trace(rtg_context* ctx, const TraceParams& p_in, cudaStream_t st, int
   const bool own = p.tally == ctx->d_tally || p.tally == ctx->d_tally_adj;
   bool ordered = own && mode != kModeLogged && wants_order(ctx, p, nrays);
   if (ordered) {
-    const uint64_t chunks = (nrays + kOrderMax - 1) / kOrderMax;
-    chunk = (nrays + chunks - 1) / chunks;
+    chunk = equal_parts(nrays, kOrderMax);
     ordered = room.take(ctx, chunk);
     if (!ordered) chunk = nrays;
   }
@@ -364,13 +379,17 @@ int launch_trace(rtg_context* ctx, const TraceParams& p_in, cudaStream_t st, int
     p.ray_begin = begin;
     p.ray_end = begin + n;
     if (ordered) {
-      const unsigned grid = (unsigned)((n + 255) / 256);
-      uint32_t* cells = room.p;
-      p.order = room.p + kCells;
-      RTG_CUDA(ctx, cudaMemsetAsync(cells, 0, kCells * sizeof(uint32_t), st));
-      order_count_kernel<<<grid, 256, 0, st>>>(p, (uint32_t)n, cells);
-      RTG_TRY(exclusive_scan_u32(ctx, cells, kCells, nullptr, st));
-      order_place_kernel<<<grid, 256, 0, st>>>(p, (uint32_t)n, cells, room.p + kCells);
+      uint32_t *cells = room.p, *order = room.p + kCells;
+      p.order = order;
+      const uint64_t piece = equal_parts(n, kOrderPiece);
+      for (uint64_t first = 0; first < n; first += piece) {
+        const uint32_t m = (uint32_t)std::min(piece, n - first);
+        const unsigned grid = (m + 255) / 256;
+        RTG_CUDA(ctx, cudaMemsetAsync(cells, 0, kCells * sizeof(uint32_t), st));
+        order_count_kernel<<<grid, 256, 0, st>>>(p, (uint32_t)first, m, cells);
+        RTG_TRY(exclusive_scan_u32(ctx, cells, kCells, nullptr, st));
+        order_place_kernel<<<grid, 256, 0, st>>>(p, (uint32_t)first, m, cells, order);
+      }
     }
     if (begin != p_in.ray_begin)
       RTG_CUDA(ctx, cudaMemsetAsync(&p.tally->next_ray, 0, sizeof(unsigned long long), st));

@@ -156,3 +156,20 @@ def test_room_is_bounded_and_given_back(rtg_lib):
         e.trace(1 << 22, 1)
         assert e.hit_counts().sum() > 0
     assert _free() >= before
+
+
+def test_room_of_a_large_launch_goes_back(rtg_lib):
+    """2^27 rays are sorted in four pieces and traced by one launch, whose ids take
+    512 MB; of these the context keeps no more than of any other launch."""
+    from rti_gb300 import Engine
+    n = (1 << 27) + 12345
+    with Engine(0) as e:
+        _deep(e)
+        e.configure(sticking=1.0)
+        e.trace(1000, 1)
+        before = _free()
+        e.trace(n, 1)
+        got = e.hit_counts(), e.tally().segments
+        assert before - _free() <= ROOM + (40 << 20)
+        assert _took_room(e, lambda: e.trace(n, 1))
+        assert np.array_equal(got[0], e.hit_counts()) and got[1] == e.tally().segments
