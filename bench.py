@@ -87,9 +87,15 @@ def read_peaks():
 
 
 def launches_per_step(rays):
-    """Kernels of one trace of the hole: path kernel and areas, and from 2^21 rays the
-    three that order the rays (count, scan, place)."""
-    return 5 if rays >= 1 << 21 else 2
+    """Kernels of one trace of the hole: a path kernel for up to 2^29 rays, the areas,
+    and from 2^21 rays three (count, scan, place) for every 2^25 of a path kernel's
+    rays, which order them."""
+    if rays < 1 << 21:
+        return 2
+    launches = -(-rays // (1 << 29))
+    share = -(-rays // launches)
+    shares = [min(share, rays - k * share) for k in range(launches)]
+    return sum(1 + 3 * -(-n // (1 << 25)) for n in shares) + 1
 
 
 def read_profile_line(key):
