@@ -206,17 +206,17 @@ RTG_API int rtg_get_tree_builder(const rtg_context* ctx, int32_t* builder);
 /* Which tree the closest-hit queries traverse (no counterpart in rti; Embree
  * chooses its own):
  *   RTG_NODES_BINARY (2): the binary tree in float boxes, visited up to four
- *     boxes at a time (128-byte nodes made by every build and refit);
+ *     boxes at a time (96-byte nodes made by every build and refit);
  *   RTG_NODES_WIDE (8): a compressed 8-wide tree collapsed from it after every
  *     build and refit (96-byte nodes, child boxes as bytes on a per-node
  *     power-of-two grid, children ordered by direction).  Its boxes contain
  *     the binary boxes, so results are the same bit for bit;
  *   RTG_NODES_AUTO (0, the default): as RTG_NODES_BINARY, the faster one on
- *     every surface measured (4.19 M discs, beyond the L2 cache, 2e7 rays:
- *     27 ms against 30.5 ms over the wide tree).
+ *     every surface measured (4.19 M discs, beyond the L2 cache, 1e7 rays:
+ *     8.2 ms against 13.3 ms over the wide tree).
  * A scene with a node wider than 4080 units, or a wide tree whose traversal
  * stack would exceed 256 entries, is traced over the binary tree whatever this
- * says.  The multi-hit window's interval queries always walk the binary tree.
+ * says.  The multi-hit window's interval queries always walk the four-box nodes.
  * rtg_autotune sets RTG_NODES_BINARY. */
 #define RTG_NODES_AUTO 0
 #define RTG_NODES_BINARY 2
@@ -286,7 +286,11 @@ RTG_API int rtg_autotune(rtg_context* ctx, uint64_t sample_rays, uint64_t seed, 
 /* Traces source rays [0, n_rays) with Philox seed `seed` on `stream`
  * (a cudaStream_t, NULL = the context's stream).  Zeroes the accumulators,
  * traces, computes the exposed areas; returns after enqueueing.  The results
- * are read with the getters below (which synchronise). */
+ * are read with the getters below (which synchronise).  A trace or adjoint replay
+ * of 2^20 rays or more may sort them by where they start, in device memory taken
+ * and given back in stream order (4 bytes a ray; the context keeps at most 128 MB
+ * of it); without room, or in a stream capture, it takes them in ascending order.
+ * The results do not depend on it but for the order of additions. */
 RTG_API int rtg_trace(rtg_context* ctx, uint64_t n_rays, uint64_t seed, void* stream);
 /* Same, for the ray range [ray_begin, ray_end) and accumulating into the
  * current totals when accumulate != 0 (used to shard rays across GPUs). */

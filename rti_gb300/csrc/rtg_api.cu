@@ -242,6 +242,7 @@ __global__ void __launch_bounds__(256) triangle_check_kernel(const uint32_t* __r
   b.reduce(c);
 }
 
+// Blocks of a grid-stride check: at most four for each of the chip's 152 SMs.
 unsigned grid_for(int64_t n) {
   const int64_t b = (n + 255) / 256;
   return (unsigned)std::max<int64_t>(1, std::min<int64_t>(b, 152 * 4));
@@ -991,14 +992,12 @@ static int rtg_autotune_body(rtg_context* ctx, uint64_t sample_rays, uint64_t se
   const int32_t keep_width = ctx->node_width;
   struct Cand {
     int32_t builder;
-    int32_t width;  // RTG_NODES_BINARY or RTG_NODES_WIDE
     rtg_launch_config lc;
     float ms;
   };
+  ctx->node_width = RTG_NODES_BINARY;  // the faster one on every surface measured
   auto run = [&](const Cand& c, float& ms) -> int {
     ctx->lc = c.lc;
-    ctx->node_width = c.width;
-    RTG_TRY(ensure_wide(ctx));
     p.s = scene_view(ctx);
     RTG_CUDA(ctx, cudaMemsetAsync(ctx->acc.p, 0, 4 * np * sizeof(double), st));
     RTG_CUDA(ctx, cudaMemsetAsync(ctx->cnt.p, 0, np * sizeof(unsigned long long), st));
@@ -1018,7 +1017,6 @@ static int rtg_autotune_body(rtg_context* ctx, uint64_t sample_rays, uint64_t se
     if (rc == RTG_OK) rc = prepare_trace(ctx, 0, sample_rays, seed, p);  // the tree changed
     if (rc != RTG_OK) break;
     const size_t first = cand.size();
-    const int32_t width = RTG_NODES_BINARY;  // the automatic choice
     // the wavefront schedule is not a candidate: its queue traffic lost to the
     // megakernel on every workload measured (it stays selectable by hand)
     for (int sched : {RTG_SCHED_MEGAKERNEL, RTG_SCHED_PLAIN})
@@ -1027,8 +1025,8 @@ static int rtg_autotune_body(rtg_context* ctx, uint64_t sample_rays, uint64_t se
           for (int stack : {0, 256}) {
             if (sched == RTG_SCHED_PLAIN && (packet != 1 || tpb == 64 || stack != 0)) continue;
             if (stack == 256 && stack_for(0, traversal_depth(ctx)) == 256) continue;
-            cand.push_back(Cand{builder, width,
-                                rtg_launch_config{tpb, packet, stack, sched, RTG_LEAF_IMMEDIATE, RTG_STACK_AUTO}, 0.0f});
+            cand.push_back(
+                Cand{builder, rtg_launch_config{tpb, packet, stack, sched, RTG_LEAF_IMMEDIATE, RTG_STACK_AUTO}, 0.0f});
           }
     float ms = 0.0f;
     for (size_t i = first; i < cand.size() && rc == RTG_OK; ++i) {
@@ -1071,7 +1069,6 @@ static int rtg_autotune_body(rtg_context* ctx, uint64_t sample_rays, uint64_t se
     if (cand[i].ms < cand[bi].ms) bi = i;
   RTG_TRY(rtg_set_tree_builder(ctx, cand[bi].builder));
   ctx->lc = cand[bi].lc;
-  ctx->node_width = cand[bi].width;
   ++ctx->version;
   if (best) *best = cand[bi].lc;
   if (best_rays_per_s) *best_rays_per_s = cand[bi].ms > 0.0f ? sample_rays / (cand[bi].ms * 1e-3) : 0.0;

@@ -510,9 +510,6 @@ void tfree(DBuf<T>& b, cudaStream_t st) {
   b.scratch = false;
 }
 
-// device helpers shared by the kernels
-__host__ __device__ inline int num_sms_hint() { return 152; }
-
 }  // namespace rtg
 
 #define RTG_CUDA(ctx, call)                                              \

@@ -532,7 +532,7 @@ __device__ float window_deposit(const TraceParams& p, f3 o, f3 d, float t0, floa
   // on the way; only a window of more than kKeep is walked again for its
   // deposits.  300 007 rays into a trench of 25 k discs: two walks over the binary
   // nodes 2.60 ms, two over the quads 2.11, one with kKeep = 16 1.70, 8 1.68.
-    constexpr int kKeep = 8;
+  constexpr int kKeep = 8;
   float kept_t[kKeep];
   int kept_id[kKeep];
   const QuadRay q = quad_ray(r);

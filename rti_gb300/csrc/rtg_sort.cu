@@ -351,7 +351,7 @@ int radix_sort_pairs(rtg_context* ctx, uint32_t* d_keys, uint32_t* d_vals, uint3
     DBuf<uint32_t> work;
     RTG_TRY(talloc(ctx, work, words, st, "radix sort"));
     cudaMemsetAsync(work.p, 0, words * sizeof(uint32_t), st);
-    const int64_t hb = (n + kRsThreads * 8 - 1) / (kRsThreads * 8);
+    const int64_t hb = (n + kRsThreads * 8 - 1) / (kRsThreads * 8);  // at most four blocks for each of 152 SMs
     rs_hist<<<(unsigned)(hb < 608 ? hb : 608), kRsThreads, 0, st>>>(d_keys, n, passes, work.p);
     uint32_t *kin = d_keys, *vin = d_vals, *kout = d_tmp_keys, *vout = d_tmp_vals;
     for (int p = 0; p < passes; ++p) {

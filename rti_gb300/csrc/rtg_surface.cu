@@ -27,7 +27,8 @@ struct Grid {
   int dim[3];
 };
 
-// Monotone in v, and off by less than 2^-23 * dim cells.
+// Monotone in v, and off by at most 3 * 2^-24 * dim cells (the roundings of the
+// difference, of inv_h and of the product).
 __device__ __forceinline__ int cell_coord(float v, float org, float inv_h, int dim) {
   const int c = (int)floorf((v - org) * inv_h);
   return c < 0 ? 0 : (c >= dim ? dim - 1 : c);

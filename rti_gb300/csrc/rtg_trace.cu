@@ -148,7 +148,9 @@ int s1_to_double(rtg_context* ctx, double* s1, int64_t n, cudaStream_t st) {
   return RTG_OK;
 }
 
-// Whether the tree and the primitive records of ctx outgrow the L2 cache.
+// Whether what the queries of ctx read outgrows the L2 cache: about 96 bytes a disc (a
+// third of the four-box nodes can be met, 32 of them; the record; the normal's basis)
+// and 128 a triangle, which is what the binary nodes and the records take.
 bool outgrows_l2(const rtg_context* ctx) {
   int l2 = 0;
   if (cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, ctx->device) != cudaSuccess) {
@@ -254,6 +256,7 @@ namespace {
 //   trench                      1e6 rays 2048 -> 2070, 2e6 3215 -> 3239, 4e6 5600 -> 5415, 1.6e7 19640 -> 19140
 //   hole, 200 k triangles       1e6 rays the same, 4e6 23200 -> 22830, 1.6e7 63170 -> 61080
 //   flat, 262 k discs           1e6 rays 790 -> 818, 4e6 2708 -> 2789, 1.6e7 10979 -> 11284: not ordered
+// (up to 4e8 rays: at kOrderPiece)
 bool wants_order(const rtg_context* ctx, const TraceParams& p, uint64_t nrays) {
   if (nrays < 1u << 20) return false;
   if (outgrows_l2(ctx)) return true;
